@@ -153,6 +153,43 @@ def test_raycast_matches_oracle(cuda_lib):
     w.destroy()
 
 
+@pytest.mark.parametrize('n, rays', [(1, 1), (255, 63), (300, 65), (1100, 4800)])
+def test_raycast_tiles_and_far_origins(cuda_lib, n, rays):
+    """Rays at the edges of the ray and body tiles, from near and from 2 km away, on long, flat and
+    unnormalised bodies: all in one call as in calls of 32, and a sample of the distances against the
+    restatement (f32 rounds a ray's offset from a body to 2^-23 of the distance, a few times over)."""
+    rng = np.random.default_rng(n)
+    scene = drop_pile(n, seed=4, spacing=1.6, layers=3)
+    for b in scene.bodies[1::3]:
+        b.size = [float(x) for x in rng.uniform(0.02, 1.5, 3)] if b.shape == 0 else b.size
+    for b in scene.bodies[1::5]:
+        b.rot = [1.3 * x for x in b.rot]
+    w = avbd_b200.CudaSolver3D(scene)
+    bodies = w.read_bodies()
+    at = bodies['pos'][rng.integers(0, n + 1, rays)] + rng.normal(0, 0.3, (rays, 3))
+    d = rng.standard_normal((rays, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    o = (at - d * rng.choice([0.0, 3.0, 2000.0], (rays, 1))).astype(np.float32)
+    d[0] = 0.0
+    hits = w.raycast(o, d)
+    parts = np.concatenate([w.raycast(o[k:k + 32], d[k:k + 32]) for k in range(0, rays, 32)])
+    assert hits.tobytes() == parts.tobytes()
+    filters = np.full((n + 1, 2), 0xFFFFFFFF, np.uint32)
+    for k in range(0, rays, max(1, rays // 40)):
+        dk = d[k].astype(np.float32).astype(float)
+        dk = (dk / (np.linalg.norm(dk) or 1.0)).astype(np.float32)
+        want = queries.raycast(bodies, None, filters, o[k], dk)
+        tol = 1e-5 * (1.0 + float(np.abs(o[k]).max()))
+        if want is None or hits['body'][k] < 0:
+            # only a ray that grazes: the other view finds it within the tolerance of a surface
+            grown = bodies.copy()
+            grown['size'] += np.float32(20 * tol)
+            assert (want is None) == (hits['body'][k] < 0) or queries.raycast(grown, None, filters, o[k], dk) is not None
+        elif hits['body'][k] == want[0]:
+            assert abs(hits['distance'][k] - want[1]) <= 20 * tol
+    w.destroy()
+
+
 def test_pose_capture_frames_match_the_world_and_round_trip(cuda_lib):
     """Pose cache frames gathered on the device every 3 steps of a pile equal the poses read back at
     those steps bit for bit, stamped with the world's step word; frames past max_frames are dropped and

@@ -76,10 +76,10 @@ struct avbd_world {
   std::string graphNote;
   std::vector<void*> allocations;
   // scratch of the queries around the step (avbd_query.cu), grown on demand: pushes, rays, the
-  // rays' nearest keys and their hits
-  float4 *pushBuf = nullptr, *rayBuf = nullptr, *rayHits = nullptr;
+  // rays' nearest keys and their hits, the bodies' spheres
+  float4 *pushBuf = nullptr, *rayBuf = nullptr, *rayHits = nullptr, *rayBounds = nullptr;
   unsigned long long* rayBest = nullptr;
-  size_t pushCap = 0, rayCap = 0, rayBestCap = 0, rayHitsCap = 0;
+  size_t pushCap = 0, rayCap = 0, rayBestCap = 0, rayHitsCap = 0, rayBoundsCap = 0;
   // hull buffer: host copy of every record (wgsl-hull.ts layout), header offsets, device capacity
   std::vector<uint32_t> hullWords;
   std::set<uint32_t> hullStarts;
