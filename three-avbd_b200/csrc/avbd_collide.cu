@@ -1509,19 +1509,16 @@ __global__ void __launch_bounds__(128) k_narrowphase(DWorld w, StepParams p) {
 // A world of a batch holds at most a few hundred bodies: its pairs are found by testing every pair
 // of bodies against the broadphase rule (the same set the grid walk finds), then collided.
 __global__ void __launch_bounds__(256) k_batch_collide(BatchLaunch B) {
-  __shared__ uint32_t s_world;
+  __shared__ WorldScope s_scope;
+  const DWorld& w = s_scope.w;
+  const StepParams& p = s_scope.p;
   for (;;) {
     __syncthreads();
-    if (threadIdx.x == 0) s_world = atomicAdd(&B.queue[0], 1u);
+    if (threadIdx.x == 0) enterWorld(B, &B.queue[0], s_scope);
     __syncthreads();
-    const uint32_t qi = s_world;
-    if (qi >= B.nWorlds) return;
-    const uint32_t wi = B.order[qi];
-    const WorldDesc d = B.worlds[wi];
-    const DWorld w = worldView(B.base, d, wi);
-    const StepParams p = worldParams(B.p, d);
+    if (s_scope.world >= B.nWorlds) return;
     uint32_t* c = w.counters;
-    const uint32_t prevPairs = min(c[C_PAIRS], d.pairCap);
+    const uint32_t prevPairs = min(c[C_PAIRS], p.pairCap);
     __syncthreads();
     if (threadIdx.x == 0) {
       c[C_PREV_PAIRS] = prevPairs;
@@ -1536,25 +1533,25 @@ __global__ void __launch_bounds__(256) k_batch_collide(BatchLaunch B) {
       c[C_ERROR] = 0;
       for (int k = 0; k < 2 * MAX_ROUND_PAIRS + 2; k++) c[C_PENDING + k] = 0;
     }
-    for (uint32_t h = threadIdx.x; h <= d.hashMask; h += blockDim.x) w.hash[h] = 0u;
+    for (uint32_t h = threadIdx.x; h <= p.hashMask; h += blockDim.x) w.hash[h] = 0u;
     __syncthreads();
     if (p.flags & FLAG_REUSE_CONTACTS)  // updateRefs, per world
-      for (uint32_t i = threadIdx.x; i < d.n; i += blockDim.x)
+      for (uint32_t i = threadIdx.x; i < p.n; i += blockDim.x)
         if (((uint32_t)w.ipos[i].w & 2u) == 0u) updateRef(w, i, c[C_STEP]);
     const int prev = 1 - p.cur;
     for (uint32_t m = threadIdx.x; m < prevPairs; m += blockDim.x) {  // hashInsert, per world
       uint4 ids = w.mIds[prev][m];
       if ((ids.w & 15u) == 0u) continue;
       if (w.ipos[ids.x].w != 0.0f || w.ipos[ids.y].w != 0.0f) continue;
-      uint32_t h = pairHash(ids.x, ids.y) & d.hashMask;
-      for (uint32_t probe = 0; probe <= d.hashMask; probe++) {
+      uint32_t h = pairHash(ids.x, ids.y) & p.hashMask;
+      for (uint32_t probe = 0; probe <= p.hashMask; probe++) {
         if (atomicCAS(&w.hash[h], 0u, m + 1u) == 0u) break;
-        h = (h + 1u) & d.hashMask;
+        h = (h + 1u) & p.hashMask;
       }
     }
     __syncthreads();
     // every pair (i > j): triangular index k -> (i, j)
-    const uint32_t n = d.n;
+    const uint32_t n = p.n;
     const uint32_t total = n * (n - 1u) / 2u;
     for (uint32_t k = threadIdx.x; k < total; k += blockDim.x) {
       uint32_t i = (uint32_t)((1.0f + sqrtf(1.0f + 8.0f * (float)k)) * 0.5f);
@@ -1573,11 +1570,11 @@ __global__ void __launch_bounds__(256) k_batch_collide(BatchLaunch B) {
     }
     __syncthreads();
     const uint32_t found = c[C_PAIRS];
-    const uint32_t pairs = min(found, d.pairCap);
+    const uint32_t pairs = min(found, p.pairCap);
     for (uint32_t pi = threadIdx.x; pi < pairs; pi += blockDim.x) narrowPair(w, p, pi);
     if (threadIdx.x == 0) {
       uint32_t bits = (c[C_OVERFLOW] & 1u) ? BATCH_OVERFLOW : 0u;
-      if (uint64_t(found) * 10u > uint64_t(d.pairCap) * 8u) bits |= BATCH_NEAR_FULL;
+      if (uint64_t(found) * 10u > uint64_t(p.pairCap) * 8u) bits |= BATCH_NEAR_FULL;
       if (bits) atomicOr(&B.status[0], bits);
     }
   }

@@ -267,6 +267,27 @@ struct BatchLaunch {
   uint32_t* status;       // [0] storage bits (BATCH_*), [1] error bits of any world
   StepParams p;           // shared parameters; per-world sizes come from the WorldDesc
 };
+// What a block (or part of one) works on: its place in the queue, past nWorlds when the queue is empty,
+// and that world's view and parameters. It lives in shared memory, written by one thread: every thread
+// keeping its own copy of the view (600 bytes, in local memory, since no thread has the registers for
+// sixty pointers) filled L1 with copies, 300 KB an SM, and put a local load before every other load
+// (4096 settled worlds, two steps and the readback: 10.75 ms, now 10.09).
+struct WorldScope {
+  uint32_t world;
+  DWorld w;
+  StepParams p;
+};
+#ifdef __CUDACC__
+__device__ inline void enterWorld(const BatchLaunch& B, uint32_t* queue, WorldScope& S) {
+  const uint32_t qi = atomicAdd(queue, 1u);
+  S.world = qi;
+  if (qi >= B.nWorlds) return;
+  const uint32_t wi = B.order[qi];
+  const WorldDesc d = B.worlds[wi];
+  S.w = worldView(B.base, d, wi);
+  S.p = worldParams(B.p, d);
+}
+#endif
 constexpr uint32_t BATCH_OVERFLOW = 1u, BATCH_NEAR_FULL = 2u;
 cudaError_t launch_batch_collision(const BatchLaunch& b, int blocks, int threads, cudaStream_t s);
 // worldThreads: 256, a block a world; 32, a warp a world (eight worlds a block)

@@ -1445,18 +1445,16 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 2) k_topology_solve(DWorld w, S
 // Batched worlds: each block takes worlds from the queue (largest first) and runs the same
 // topology + solve code for one world at block scope.
 __global__ void __launch_bounds__(SOLVE_THREADS, 2) k_batch_solve(BatchLaunch B) {
-  __shared__ uint32_t s_world;
+  __shared__ WorldScope s_scope;
+  const WorldScope& S = s_scope;
+  const DWorld& w = S.w;
+  const StepParams& p = S.p;
   for (;;) {
     __syncthreads();
-    if (threadIdx.x == 0) s_world = atomicAdd(&B.queue[1], 1u);
+    if (threadIdx.x == 0) enterWorld(B, &B.queue[1], s_scope);
     __syncthreads();
-    const uint32_t qi = s_world;
-    if (qi >= B.nWorlds) return;
-    const uint32_t wi = B.order[qi];
-    const WorldDesc d = B.worlds[wi];
-    const DWorld w = worldView(B.base, d, wi);
-    const StepParams p = worldParams(B.p, d);
-    for (uint32_t i = threadIdx.x; i <= d.n; i += SOLVE_THREADS) {
+    if (S.world >= B.nWorlds) return;
+    for (uint32_t i = threadIdx.x; i <= p.n; i += SOLVE_THREADS) {
       w.adjStart[i] = 0u;
       w.adjFill[i] = 0u;
     }
@@ -1478,17 +1476,15 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 2) k_batch_solve_sub(BatchLaunc
   using Team = SubTeam<kT>;
   Team team;
   const uint32_t r = team.rank();
-  __shared__ uint32_t s_next[Team::kUnits];
+  __shared__ WorldScope s_scope[Team::kUnits];
+  const WorldScope& S = s_scope[team.unit()];
+  const DWorld& w = S.w;
+  const StepParams& p = S.p;
   for (;;) {
-    if (r == 0) s_next[team.unit()] = atomicAdd(&B.queue[1], 1u);
+    if (r == 0) enterWorld(B, &B.queue[1], s_scope[team.unit()]);
     team.lsync();
-    const uint32_t qi = s_next[team.unit()];
-    if (qi >= B.nWorlds) return;
-    const uint32_t wi = B.order[qi];
-    const WorldDesc d = B.worlds[wi];
-    const DWorld w = worldView(B.base, d, wi);
-    const StepParams p = worldParams(B.p, d);
-    for (uint32_t i = r; i <= d.n; i += kT) {
+    if (S.world >= B.nWorlds) return;
+    for (uint32_t i = r; i <= p.n; i += kT) {
       w.adjStart[i] = 0u;
       w.adjFill[i] = 0u;
     }
