@@ -316,7 +316,7 @@ int avbd_read_phase_clocks(avbd_world* world, double* dst, uint32_t cap, uint32_
 /* Steps replay a captured CUDA graph (default on; per-step statistics launch directly). */
 int avbd_use_graphs(avbd_world* world, int enable);
 
-/* Blocks of the cooperative topology + solve launch (0: every co-resident block, the default). The
+/* Blocks of the cooperative topology + solve launch (0: by the world's size, the default). The
  * lane groups a body's rows are summed in depend on the launch's thread count, so results differ in
  * the last bits between launch shapes; one block reproduces a batched world's step bit for bit. */
 int avbd_set_solve_blocks(avbd_world* world, int blocks);

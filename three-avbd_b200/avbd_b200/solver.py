@@ -438,7 +438,7 @@ class CudaSolver3D:
         self._check(self.lib.avbd_use_graphs(self.handle, 1 if on else 0))
 
     def set_solve_blocks(self, blocks: int = 0):
-        """Blocks of the cooperative topology + solve launch (0: all co-resident ones)."""
+        """Blocks of the cooperative topology + solve launch (0: by the world's size)."""
         self._check(self.lib.avbd_set_solve_blocks(self.handle, blocks))
 
     def enable_step_stats(self, capacity: int):

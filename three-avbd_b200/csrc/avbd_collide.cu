@@ -124,10 +124,24 @@ __device__ __forceinline__ void countManifold(const DWorld& w, uint32_t count) {
   }
 }
 
+// A point's penalty and multiplier words with C0's tangential parts: in the record where the contact
+// layout has them, or, for the dataflow sweep, beside it with tag 0 in their place (the sweep's last
+// update of the point puts them back)
+template <bool kFlow>
+__device__ __forceinline__ void storePoint(const DWorld& w, uint32_t slot, float4* o, float3 pen, float3 lam, float c0y, float c0z, bool swept) {
+  if (kFlow && swept) {
+    w.c0t[slot] = make_float2(c0y, c0z);
+    c0y = c0z = 0.0f;
+  }
+  o[K_PEN] = make_float4(pen.x, pen.y, pen.z, c0y);
+  o[K_LAM] = make_float4(lam.x, lam.y, lam.z, c0z);
+}
+
 // copyContacts (wgsl-collision.ts:721-753): last step's manifold in slot pm kept as this step's
 // manifold in slot pi (ids with its generation step, normal, friction, points with their keys and
 // anchors), each point's C(x-) evaluated at the current poses and its multipliers and penalties
 // warm-started as a fresh point's are
+template <bool kFlow>
 __device__ void copyContacts(const DWorld& w, const StepParams& p, uint32_t pi, uint32_t pm) {
   const int cur = p.cur, prev = 1 - cur;
   const uint4 ids = w.mIds[prev][pm];
@@ -142,6 +156,8 @@ __device__ void copyContacts(const DWorld& w, const StepParams& p, uint32_t pi, 
   const float3 cA = f3(w.pos[a]), cB = f3(w.pos[b]);
   const float4 qA = w.rot[a], qB = w.rot[b];
   const float penaltyMin = contactPenaltyMin(w, p, a, b);
+  // kept manifolds may hold pairs without a moving body any more, which no sweep updates
+  const bool swept = kFlow && p.iterations > 0 && ((enabled(w, a) && w.size[a].w > 0.0f) || (enabled(w, b) && w.size[b].w > 0.0f));
   for (uint32_t i = 0; i < count; i++) {
     const float4* q = w.cPt[prev] + 4 * (size_t(ids.z) + i);
     const float4 ra = q[K_RA], rb = q[K_RB];
@@ -152,23 +168,24 @@ __device__ void copyContacts(const DWorld& w, const StepParams& p, uint32_t pi, 
     pen = make_float3(fminf(fmaxf(pen.x * p.gamma, PENALTY_MIN), PENALTY_MAX), fminf(fmaxf(pen.y * p.gamma, PENALTY_MIN), PENALTY_MAX),
                       fminf(fmaxf(pen.z * p.gamma, PENALTY_MIN), PENALTY_MAX));
     pen.x = fmaxf(pen.x, penaltyMin);
-    float4* o = w.cPt[cur] + 4 * (size_t(pi) * MAX_CONTACTS + i);
+    const size_t slot = size_t(pi) * MAX_CONTACTS + i;
+    float4* o = w.cPt[cur] + 4 * slot;
     o[K_RA] = ra;
     o[K_RB] = make_float4(rb.x, rb.y, rb.z, c0x);
-    o[K_PEN] = make_float4(pen.x, pen.y, pen.z, c0y);
-    o[K_LAM] = make_float4(lam.x, lam.y, lam.z, c0z);
+    storePoint<kFlow>(w, uint32_t(slot), o, pen, lam, c0y, c0z, swept);
   }
 }
 
 // reuseContacts (wgsl-collision.ts:706-717): the pair keeps last step's points when they were
 // generated no earlier than either body's last move
+template <bool kFlow>
 __device__ inline bool reusePair(const DWorld& w, const StepParams& p, uint32_t pi, uint32_t a, uint32_t b) {
   const int pm = hashFind(w, p, a, b);
   if (pm < 0) return false;
   const uint32_t idw = w.mIds[1 - p.cur][pm].w;
   const uint32_t moved = max(__float_as_uint(w.ypos[a].w), __float_as_uint(w.ypos[b].w));
   if ((idw & 15u) == 0u || (idw >> 4) < moved) return false;
-  copyContacts(w, p, pi, (uint32_t)pm);
+  copyContacts<kFlow>(w, p, pi, (uint32_t)pm);
   return true;
 }
 
@@ -185,7 +202,7 @@ __global__ void k_reuse_manifolds(DWorld w, StepParams p) {
       w.mIds[p.cur][m] = make_uint4(ids.x, ids.y, m * MAX_CONTACTS, ids.w & ~15u);
       continue;
     }
-    copyContacts(w, p, m, m);
+    copyContacts<true>(w, p, m, m);
   }
 }
 
@@ -1349,9 +1366,12 @@ __device__ void collidePolyWarp(const DWorld& w, const Poly& A, const Poly& B, b
   hullFaceContact(w, A, B, true, faFace, found);
 }
 
+template <bool kFlow>
 __device__ __forceinline__ void writeManifold(const DWorld& w, const StepParams& p, uint32_t pi, uint32_t a, uint32_t b, const Box& A, const Box& B, const Sat& sat,
                               const Found& found, bool anySphere);
 
+// kFlow: a single world, whose dataflow sweep takes its points' words as storePoint lays them out
+template <bool kFlow>
 __device__ void narrowPair(const DWorld& w, const StepParams& p, uint32_t pi) {
   {
     uint2 pr = w.pairs[pi];
@@ -1362,7 +1382,7 @@ __device__ void narrowPair(const DWorld& w, const StepParams& p, uint32_t pi) {
     sat.valid = false;
     Found found;
     found.count = 0;
-    if ((p.flags & FLAG_REUSE_CONTACTS) && reusePair(w, p, pi, a, b)) return;
+    if ((p.flags & FLAG_REUSE_CONTACTS) && reusePair<kFlow>(w, p, pi, a, b)) return;
     bool sphereA = w.avel[a].w == SHAPE_SPHERE_F, sphereB = w.avel[b].w == SHAPE_SPHERE_F;
     float4 qA = w.rot[a], qB = w.rot[b];
     if (sphereA && sphereB) {
@@ -1398,12 +1418,13 @@ __device__ void narrowPair(const DWorld& w, const StepParams& p, uint32_t pi) {
     } else {
       collideBoxes(A, B, (p.flags & FLAG_FACE_BIAS) != 0u, sat, found);
     }
-    writeManifold(w, p, pi, a, b, A, B, sat, found, sphereA || sphereB);
+    writeManifold<kFlow>(w, p, pi, a, b, A, B, sat, found, sphereA || sphereB);
   }
 }
 
 // Pair slot pi's manifold from its contacts: ids, normal and friction, and every point warm-started
 // from last step's point of the same feature (wgsl-collision.ts:812-900)
+template <bool kFlow>
 __device__ __forceinline__ void writeManifold(const DWorld& w, const StepParams& p, uint32_t pi, uint32_t a, uint32_t b, const Box& A, const Box& B, const Sat& sat,
                               const Found& found, bool anySphere) {
   const int cur = p.cur, prev = 1 - cur;
@@ -1474,8 +1495,7 @@ __device__ __forceinline__ void writeManifold(const DWorld& w, const StepParams&
       float4* o = w.cPt[cur] + 4 * slot;
       o[K_RA] = make_float4(rA.x, rA.y, rA.z, __uint_as_float(found.feature[i] | stick));
       o[K_RB] = make_float4(rB.x, rB.y, rB.z, c0x);
-      o[K_PEN] = make_float4(pen.x, pen.y, pen.z, c0y);
-      o[K_LAM] = make_float4(lam.x, lam.y, lam.z, c0z);
+      storePoint<kFlow>(w, slot, o, pen, lam, c0y, c0z, p.iterations > 0);
     }
   }
 }
@@ -1494,7 +1514,7 @@ __global__ void __launch_bounds__(256) k_hull_narrowphase(DWorld w, StepParams p
     Found found;
     found.count = 0;
     collidePolyWarp(w, polyOf(w, pr.x), polyOf(w, pr.y), (p.flags & FLAG_FACE_BIAS) != 0u, lane, sat, found);
-    if (lane == 0u) writeManifold(w, p, pi, pr.x, pr.y, makeBox(w, pr.x), makeBox(w, pr.y), sat, found, false);
+    if (lane == 0u) writeManifold<true>(w, p, pi, pr.x, pr.y, makeBox(w, pr.x), makeBox(w, pr.y), sat, found, false);
     __syncwarp();
   }
 }
@@ -1502,7 +1522,7 @@ __global__ void __launch_bounds__(256) k_hull_narrowphase(DWorld w, StepParams p
 __global__ void __launch_bounds__(128) k_narrowphase(DWorld w, StepParams p) {
   uint32_t total = w.counters[C_PAIRS];
   if (total > p.pairCap) total = p.pairCap;
-  for (uint32_t pi = blockIdx.x * blockDim.x + threadIdx.x; pi < total; pi += gridDim.x * blockDim.x) narrowPair(w, p, pi);
+  for (uint32_t pi = blockIdx.x * blockDim.x + threadIdx.x; pi < total; pi += gridDim.x * blockDim.x) narrowPair<true>(w, p, pi);
 }
 
 // --- batched worlds: one block per world ------------------------------------------------------------------
@@ -1571,7 +1591,7 @@ __global__ void __launch_bounds__(256) k_batch_collide(BatchLaunch B) {
     __syncthreads();
     const uint32_t found = c[C_PAIRS];
     const uint32_t pairs = min(found, p.pairCap);
-    for (uint32_t pi = threadIdx.x; pi < pairs; pi += blockDim.x) narrowPair(w, p, pi);
+    for (uint32_t pi = threadIdx.x; pi < pairs; pi += blockDim.x) narrowPair<false>(w, p, pi);
     if (threadIdx.x == 0) {
       uint32_t bits = (c[C_OVERFLOW] & 1u) ? BATCH_OVERFLOW : 0u;
       if (uint64_t(found) * 10u > uint64_t(p.pairCap) * 8u) bits |= BATCH_NEAR_FULL;

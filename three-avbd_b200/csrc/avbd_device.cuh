@@ -71,6 +71,7 @@ struct StepParams {
   uint32_t step;
   uint32_t fixedColors;  // colours come from the host (validation), no Jones-Plassmann
   uint32_t colorCap;
+  uint32_t laneBudget;   // threads the grid's lane classes are sized by (0: the launch's own)
   uint32_t rowsPerLane;  // the least rows a lane of a body's group takes (0, 1: as the colour's size asks)
   int cur;               // which manifold/contact buffers this step writes
 };
@@ -107,14 +108,15 @@ struct DWorld {
   uint32_t *colorA, *colorB, *colorHist, *colorStart, *colorBodies, *fixedColor;
   uint32_t *incCount, *incStart;
   uint2* incList;         // per incidence: constraint row (joint slot, or nj + point slot) | OWNER_BIT, partner word
-  uint32_t* done;         // per body: iterations finished in this step's dataflow sweep (pose and owned rows)
-  uint32_t* poseDone;     // per body: iterations whose pose is written (published before its owned rows)
+  float2* c0t;            // per point slot: C0 along t1 and t2, whose place in the point's record the dataflow sweep's tags take (null: batched worlds)
+  float4* words;          // per body: the dataflow sweep's four tagged words (its pose since x-)
+  uint32_t* done;         // per body: iterations after which the joints it updates are written
   uint4* laneTable;       // per lane of the dataflow sweep: body, first row, row end, L | sub << 8
   uint32_t* bucket;       // BUCKET_WORDS: counts, starts (+ total), fill cursors, lane bases, lane totals per colour
   // Per body, the step's unknowns relative to x- (kept by the solve, precise at any distance from the
   // origin, where an absolute f32 position rounds to its magnitude's ulp): dlin = x - x- and
   // dang = (2 vec(r), r.w) with r the rotation since x- (q = r q-, so qsub(q, q-) = dang.xyz); and
-  // the inertial target y the same way: ylin = y - x-, yang = the rotation from q- to y's rotation.
+  // the inertial target y the same way: ylin = y - x-, yang = the rotation from q- to y's rotation. The dataflow sweep keeps its poses in `words` instead of dlin and dang.
   float4 *dlin, *dang, *ylin, *yang;
   // contact reuse (wgsl-collision.ts:20-44): per body its reference pose (zero rotation: none yet);
   // the step it last moved past the tolerances is kept in ypos.w (the record's moved_step word)
@@ -165,6 +167,8 @@ __host__ __device__ inline DWorld worldView(const DWorld& b, const WorldDesc& d,
   v.colorBodies += d.body;
   v.fixedColor += d.body;
   v.done = nullptr;
+  v.c0t = nullptr;
+  v.words = nullptr;
   v.laneTable = nullptr;
   v.incCount += d.body;
   v.incStart += d.body + wi;
@@ -326,6 +330,6 @@ cudaError_t launch_record_step(const BatchLaunch& L, const RecordDev& R, uint32_
 
 // Host launchers (avbd_solve.cu)
 int solve_grid_blocks(int device);
-cudaError_t launch_topology_solve(const DWorld& w, const StepParams& p, int blocks, cudaStream_t s);
+cudaError_t launch_topology_solve(const DWorld& w, const StepParams& p, int blocks, int maxBlocks, int sms, cudaStream_t s);
 
 }  // namespace avbd

@@ -137,6 +137,7 @@ int allocPairs(avbd_world* w, uint32_t cap) {
   dfree(w, d.incList);
   dfree(w, d.laneTable);
   dfree(w, d.hullPairs);
+  dfree(w, d.c0t);
   w->pairCap = cap;
   w->configGen++;
   w->hashSize = pow2AtLeast(2ull * cap);
@@ -144,6 +145,7 @@ int allocPairs(avbd_world* w, uint32_t cap) {
   w->incCap = 2u * (cap * MAX_CONTACTS + w->jointCap);
   CUDA_TRY(w, dalloc(w, &d.pairs, cap));
   CUDA_TRY(w, dalloc(w, &d.hullPairs, cap));
+  CUDA_TRY(w, dalloc(w, &d.c0t, size_t(cap) * MAX_CONTACTS));
   CUDA_TRY(w, dalloc(w, &d.hash, w->hashSize));
   CUDA_TRY(w, dalloc(w, &d.adjList, w->adjCap));
   CUDA_TRY(w, dalloc(w, &d.incList, w->incCap));
@@ -433,7 +435,8 @@ int avbd_world_create(const avbd_config* cfg, avbd_world** out) {
   const uint32_t B = w->bodyCap;
   w->tableSize = pow2AtLeast(2ull * B);
   w->sortTiles = (B + 8191) / 8192;
-  w->solveBlocks = w->maxSolveBlocks = solve_grid_blocks(w->device);
+  w->maxSolveBlocks = solve_grid_blocks(w->device);
+  w->sms = prop.multiProcessorCount;
   bool ok = true;
   auto A = [&](cudaError_t e) { ok = ok && e == cudaSuccess; };
   for (float4** f : {&d.pos, &d.rot, &d.ipos, &d.irot, &d.size, &d.moment, &d.ypos, &d.yrot, &d.vel, &d.avel}) A(dalloc(w, f, B));
@@ -460,22 +463,20 @@ int avbd_world_create(const avbd_config* cfg, avbd_world** out) {
   A(dalloc(w, &d.adjFill, B + 1));
   A(dalloc(w, &d.colorA, B));
   A(dalloc(w, &d.colorB, B));
-  A(dalloc(w, &d.colorHist, size_t(MAX_COLORS) * w->solveBlocks + 1));
+  A(dalloc(w, &d.colorHist, size_t(MAX_COLORS) * w->maxSolveBlocks + 1));
   A(dalloc(w, &d.colorStart, MAX_COLORS + 1));
   A(dalloc(w, &d.colorBodies, B));
   A(dalloc(w, &d.fixedColor, B));
   A(dalloc(w, &d.incStart, B + 1));
   A(dalloc(w, &d.incCount, B));
   A(dalloc(w, &d.bucket, BUCKET_WORDS));
-  A(dalloc(w, &d.dlin, B));
-  A(dalloc(w, &d.dang, B));
   A(dalloc(w, &d.ylin, B));
   A(dalloc(w, &d.yang, B));
   A(dalloc(w, &d.refPos, B));
   A(dalloc(w, &d.refRot, B));
   A(dalloc(w, &d.done, B));
-  A(dalloc(w, &d.poseDone, B));
-  A(dalloc(w, &d.scanScratch, w->solveBlocks + 1));
+  A(dalloc(w, &d.words, size_t(B) * 4));
+  A(dalloc(w, &d.scanScratch, w->maxSolveBlocks + 1));
   A(dalloc(w, &d.counters, COUNTER_WORDS));
   A(dalloc(w, &d.barrier, 2));
   A(dalloc(w, &d.clocks, CLOCK_WORDS));
@@ -963,7 +964,7 @@ int avbd_step_with(avbd_world* w, int n, const avbd_step_options* opts) {
     StepParams p = makeParams(w);
     auto enqueue = [&]() -> cudaError_t {
       uint32_t launches = launch_collision(w->d, p, w->tableSize, reuse, w->stream) + 1;
-      cudaError_t le = launch_topology_solve(w->d, p, w->solveBlocks, w->stream);
+      cudaError_t le = launch_topology_solve(w->d, p, w->solveBlocks, w->maxSolveBlocks, w->sms, w->stream);
       if (w->statsCap) launch_step_stats(w->d, launches + 1, w->stream);
       w->launchesPerStep = launches + (w->statsCap ? 1 : 0);
       cudaMemcpyAsync(w->hCounters, w->d.counters, COUNTER_WORDS * sizeof(uint32_t), cudaMemcpyDeviceToHost, w->stream);
@@ -1252,7 +1253,7 @@ int avbd_use_graphs(avbd_world* w, int enable) {
 int avbd_set_solve_blocks(avbd_world* w, int blocks) {
   if (!w || blocks < 0) return AVBD_ERR_INVALID;
   if (blocks > w->maxSolveBlocks) return fail(w, AVBD_ERR_INVALID, "at most " + std::to_string(w->maxSolveBlocks) + " co-resident solve blocks");
-  w->solveBlocks = blocks ? blocks : w->maxSolveBlocks;
+  w->solveBlocks = blocks;
   w->configGen++;
   return AVBD_OK;
 }

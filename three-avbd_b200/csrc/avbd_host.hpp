@@ -43,7 +43,7 @@ struct avbd_world {
   uint32_t sortTiles = 0;
   DWorld d{};
   float4* staging = nullptr;  // body records for host transfers (10 float4 a body, capacity)
-  int solveBlocks = 0, maxSolveBlocks = 0;  // the cooperative solve's grid (maxSolveBlocks: all co-resident)
+  int solveBlocks = 0, maxSolveBlocks = 0, sms = 0;  // the cooperative solve's grid (0: by the world's size; maxSolveBlocks: all co-resident)
   int cur = 0;
   uint32_t stepCount = 0;
   bool fixedColors = false;

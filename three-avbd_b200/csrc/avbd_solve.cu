@@ -17,6 +17,8 @@
 // iteration nothing reads its multipliers until the next iteration, so updating it there equals
 // the reference's separate dual pass after every colour (solver.ts:2246-2259), with one grid
 // barrier per iteration fewer and the contact rows still in cache.
+#include <algorithm>
+
 #include "avbd_device.cuh"
 
 namespace avbd {
@@ -33,9 +35,9 @@ __device__ __forceinline__ unsigned long long globaltimer() {
   return t;
 }
 
-__device__ __forceinline__ uint32_t atom_add_release_gpu(uint32_t* p, uint32_t v) {
+__device__ __forceinline__ uint32_t atom_add_acq_rel_gpu(uint32_t* p, uint32_t v) {
   uint32_t old;
-  asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
   return old;
 }
 __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
@@ -45,8 +47,9 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
 }
 
 // Grid barrier: a monotonic arrival counter (zeroed before the launch); the k-th barrier completes
-// when it reaches k x gridDim.x. Arrival is a release, the wait an acquire (PTX memory model), so
-// every block's writes before the barrier are visible to every block after it. The wait is bounded:
+// when it reaches k x gridDim.x. Arrival is a release, the wait an acquire (PTX memory model), and
+// arrival an acquire too, for the block that arrives last and does not wait: every block's writes
+// before the barrier are visible to every block after it. The wait is bounded:
 // past the clock budget the block sets an error bit and returns false, and every other block
 // leaves at its next wait. The last block to arrive stamps the device time for the phase profile.
 __device__ unsigned long long* g_clocks;
@@ -57,7 +60,7 @@ __device__ bool grid_sync(uint32_t* bar, uint32_t* counters) {
   if (threadIdx.x == 0) {
     uint32_t target = (++s_epoch) * gridDim.x;
     uint32_t ab = 0;
-    uint32_t old = atom_add_release_gpu(bar, 1u);
+    uint32_t old = atom_add_acq_rel_gpu(bar, 1u);
     if (old + 1u == target) {
       unsigned long long* ck = g_clocks;
       if (ck) {
@@ -69,6 +72,7 @@ __device__ bool grid_sync(uint32_t* bar, uint32_t* counters) {
       }
     } else {
       long long t0 = clock64();
+      uint32_t polls = 0;
       while (ld_acquire_gpu(bar) < target) {
         if (ldv(&counters[C_ERROR]) & (ERR_BARRIER_TIMEOUT | ERR_DEPENDENCY_TIMEOUT)) { ab = 1; break; }
         if (clock64() - t0 > BARRIER_CYCLES) {
@@ -76,7 +80,7 @@ __device__ bool grid_sync(uint32_t* bar, uint32_t* counters) {
           ab = 1;
           break;
         }
-        __nanosleep(32);
+        if (++polls > 64u) __nanosleep(32);
       }
     }
     s_abort = ab;
@@ -144,12 +148,14 @@ __device__ uint32_t warp_scan_range(uint32_t* data, uint32_t lo, uint32_t hi) {
 // (one small world of a batch on a warp, two or four warps, SubTeam). A team's "unit" is the part of
 // it that shares one copy of the shared-memory tables: a block, or a sub-block team itself.
 // laneBudget is the thread count the lane classes are sized by: a sub-block team sizes them as a
-// block does, so that every body gets the same lanes and sums its rows in the same order.
+// block does, and a grid launch of fewer blocks than fit as the full one does, so that every body gets
+// the same lanes and sums its rows in the same order.
 struct GridTeam {
   static constexpr bool kDataflow = true;  // colour passes as a dataflow sweep (no grid barrier per colour)
   static constexpr uint32_t kUnits = 1;
   uint32_t* bar;
   uint32_t* ctr;
+  uint32_t budget;  // 0: the launch's own threads
   __device__ uint32_t rank() const { return blockIdx.x * blockDim.x + threadIdx.x; }
   __device__ uint32_t size() const { return gridDim.x * blockDim.x; }
   __device__ uint32_t block() const { return blockIdx.x; }
@@ -160,7 +166,7 @@ struct GridTeam {
   __device__ uint32_t lsize() const { return blockDim.x; }
   __device__ void lsync() const { __syncthreads(); }
   __device__ uint32_t scan(uint32_t* data, uint32_t lo, uint32_t hi) const { return block_scan_range(data, lo, hi); }
-  __device__ uint32_t laneBudget() const { return size(); }
+  __device__ uint32_t laneBudget() const { return budget ? budget : size(); }
 };
 struct BlockTeam {
   static constexpr bool kDataflow = false;  // a block's __syncthreads per colour costs little
@@ -449,18 +455,31 @@ struct Bodies2 {
   uint32_t own;
   const Pose* ownPose;
   bool atStart;
+  static constexpr bool kShared = false;
   __device__ inline float3 base(int i) const { return atStart ? f3(w->pos[i]) : (uint32_t)i == own ? ownPose->x0 : f3(w->ipos[i]); }
   __device__ inline float3 disp(int i) const {
     return atStart ? make_float3(0.0f, 0.0f, 0.0f) : (uint32_t)i == own ? ownPose->dLin : f3(w->dlin[i]);
   }
   __device__ inline float4 rot(int i) const { return (uint32_t)i == own ? ownPose->q : w->rot[i]; }
 };
-__device__ inline float3 jointLinC(const float4* k, int a, int b, const Bodies2& B) {
+// The same with both bodies' poses in registers, as the dataflow sweep has them; the joint's record is
+// then read past L1, where another SM's update of it would not show
+struct PosePair {
+  uint32_t own;
+  const Pose *ownPose, *other;
+  static constexpr bool kShared = true;
+  __device__ inline float3 base(int i) const { return (uint32_t)i == own ? ownPose->x0 : other->x0; }
+  __device__ inline float3 disp(int i) const { return (uint32_t)i == own ? ownPose->dLin : other->dLin; }
+  __device__ inline float4 rot(int i) const { return (uint32_t)i == own ? ownPose->q : other->q; }
+};
+template <class Bodies>
+__device__ inline float3 jointLinC(const float4* k, int a, int b, const Bodies& B) {
   float3 rb = qrotate(B.rot(b), f3(k[J_RB]));
   if (a < 0) return ((f3(k[J_RA]) - B.base(b)) - B.disp(b)) - rb;  // a world point against body b
   return ((B.base(a) - B.base(b)) + (B.disp(a) - B.disp(b))) + (qrotate(B.rot(a), f3(k[J_RA])) - rb);
 }
-__device__ inline float3 jointAngC(const float4* k, int a, int b, const Bodies2& B) {
+template <class Bodies>
+__device__ inline float3 jointAngC(const float4* k, int a, int b, const Bodies& B) {
   float4 qb = B.rot(b);
   float4 ra = a < 0 ? make_float4(0.0f, 0.0f, 0.0f, 1.0f) : B.rot(a);
   float l = ((qb.x * qb.x + qb.y * qb.y) + qb.z * qb.z) + qb.w * qb.w;
@@ -470,16 +489,18 @@ __device__ inline float3 jointAngC(const float4* k, int a, int b, const Bodies2&
   float s = 2.0f * k[J_LAM_ANG].w;
   return make_float3(d.x * s, d.y * s, d.z * s);
 }
+template <bool kShared>
 __device__ inline void loadJoint(const DWorld& w, uint32_t j, float4* k) {
 #pragma unroll
-  for (int i = 0; i < JOINT_VEC4; i++) k[i] = w.joint[j * JOINT_VEC4 + i];
+  for (int i = 0; i < JOINT_VEC4; i++) k[i] = kShared ? __ldcg(w.joint + (j * JOINT_VEC4 + i)) : w.joint[j * JOINT_VEC4 + i];
 }
 
-__device__ void addJoint(Acc& acc, const DWorld& w, uint32_t j, float alpha, uint32_t i, const Bodies2& B) {
+template <class Bodies>
+__device__ void addJoint(Acc& acc, const DWorld& w, uint32_t j, float alpha, uint32_t i, const Bodies& B) {
   int4 info = w.jinfo[j];
   int a = info.y, b = info.z;
   float4 k[JOINT_VEC4];
-  loadJoint(w, j, k);
+  loadJoint<Bodies::kShared>(w, j, k);
   bool isA = (int)i == a;
   float sg = isA ? 1.0f : -1.0f;
   if ((uint32_t)info.x == T_SPRING) {
@@ -521,12 +542,13 @@ __device__ void addJoint(Acc& acc, const DWorld& w, uint32_t j, float alpha, uin
   }
 }
 
-__device__ void dualJoint(const DWorld& w, const StepParams& p, uint32_t j, const Bodies2& B) {
+template <class Bodies>
+__device__ void dualJoint(const DWorld& w, const StepParams& p, uint32_t j, const Bodies& B) {
   int4 info = w.jinfo[j];
   if ((uint32_t)info.x != T_JOINT) return;
   int a = info.y, b = info.z;
   float4 k[JOINT_VEC4];
-  loadJoint(w, j, k);
+  loadJoint<Bodies::kShared>(w, j, k);
   const float alpha = p.alpha;
   float4 penLin = k[J_PEN_LIN], penAng = k[J_PEN_ANG], lamLin = k[J_LAM_LIN], lamAng = k[J_LAM_ANG];
   if (dot3(f3(penLin), f3(penLin)) > 0.0f) {
@@ -645,6 +667,13 @@ struct PointView {
   bool isA;
   Pose other;
 };
+__device__ __forceinline__ void viewPoint(const DWorld& w, float4 geo, uint32_t i, uint32_t partner, PointView& v) {
+  v.n = f3(geo);
+  v.friction = geo.w;
+  orthonormal(v.n, v.t1, v.t2);
+  v.isA = i > partner;  // a pair's A is its higher index
+  if ((__float_as_uint(v.ra.w) & ~STICK_BIT) == SPHERE_FEATURE) v.other.q0 = w.irot[partner];
+}
 __device__ inline void loadPoint(const DWorld& w, const StepParams& p, uint32_t cs, uint32_t i, uint32_t partner, PointView& v) {
   const float4* pt = w.cPt[p.cur] + 4 * cs;
   v.ra = pt[K_RA];
@@ -658,6 +687,33 @@ __device__ inline void loadPoint(const DWorld& w, const StepParams& p, uint32_t 
   v.isA = i > partner;  // a pair's A is its higher index
   v.other = partnerPose(w, partner);
   if ((__float_as_uint(v.ra.w) & ~STICK_BIT) == SPHERE_FEATURE) v.other.q0 = w.irot[partner];
+}
+
+__device__ __forceinline__ void evalPoint(const PointView& v, const Pose& own, float alpha, ContactEval& e) {
+  const Pose& A = v.isA ? own : v.other;
+  const Pose& B = v.isA ? v.other : own;
+  evalContact(v.ra, v.rb, v.pen, v.lam, v.n, v.t1, v.t2, v.friction, A, B, alpha, e);
+}
+__device__ __forceinline__ void addView(Acc& acc, const PointView& v, const Pose& own, float alpha) {
+  ContactEval e;
+  evalPoint(v, own, alpha, e);
+  addPoint(acc, v.isA ? e.rAW : e.rBW, v.n, v.t1, v.t2, make_float3(v.pen.x, v.pen.y, v.pen.z), e.F, v.isA ? 1.0f : -1.0f);
+}
+// The dual update of a point (wgsl-solve.ts:637-662): its new multipliers and penalties (the words' w
+// kept) and key
+__device__ __forceinline__ void dualView(const PointView& v, const Pose& own, const StepParams& p, float4& pen, float4& lam, uint32_t& key) {
+  ContactEval e;
+  evalPoint(v, own, p.alpha, e);
+  lam = make_float4(e.F.x, e.F.y, e.F.z, v.lam.w);
+  pen = v.pen;
+  key = __float_as_uint(v.ra.w);
+  if (e.F.x < 0.0f) pen.x = fminf(pen.x + p.betaLin * fabsf(e.C.x), PENALTY_MAX);
+  if (e.frictionScale <= e.bounds) {
+    pen.y = fminf(pen.y + p.betaLin * fabsf(e.C.y), PENALTY_MAX);
+    pen.z = fminf(pen.z + p.betaLin * fabsf(e.C.z), PENALTY_MAX);
+    bool stick = sqrtf(e.C.y * e.C.y + e.C.z * e.C.z) < STICK_THRESH;
+    key = (key & ~STICK_BIT) | (stick ? STICK_BIT : 0u);
+  }
 }
 
 __device__ inline void accumulateIncidence(Acc& acc, const DWorld& w, const StepParams& p, uint2 inc, uint32_t i, const Pose& own) {
@@ -720,15 +776,50 @@ constexpr int B_COUNT = 0, B_START = BUCKETS, B_FILL = 2 * BUCKETS + 1, B_LANE =
               B_ROWS = B_LANE_TOTAL + MAX_COLORS;
 static_assert(B_ROWS + MAX_COLORS <= BUCKET_WORDS, "bucket words");
 
-// Waits until a body's count (`flag`: its done or poseDone word, published with release semantics)
-// reaches `need`. Bounded: past the clock budget, or once any wait of the launch gave up, it returns
-// false.
-__device__ inline bool waitDone(const DWorld& w, const uint32_t* flag, uint32_t need) {
-  if (ld_acquire_gpu(flag) >= need) return true;
-  const long long t0 = clock64();
-  for (uint32_t n = 1;; n++) {
+// --- the dataflow sweep's words -----------------------------------------------------------------------------
+// A word of the sweep is 16 bytes, three values and in w a tag, the iterations whose result it holds,
+// written and read by single 128-bit accesses (each atomic as a whole): a reader polls the word itself
+// until its tag says that it is the wanted one, so a result needs no flag, no fence before it and no
+// second round trip to L2 after it. The sweep is a chain of colours times iterations, each link as long
+// as it takes one body's result to reach the next: with a release store of a count and acquire loads of
+// it, which also emptied L1 of the rows' fixed parts each time, 48 boxes took 127 us of sweep, 3001
+// bodies 231 and 100000 1155; with tagged words 96, 141 and 998 (a B200, 10 iterations).
+__device__ __forceinline__ float4 ldWord(const float4* p) {
+  unsigned long long lo, hi;
+  asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+  return make_float4(__uint_as_float(uint32_t(lo)), __uint_as_float(uint32_t(lo >> 32)), __uint_as_float(uint32_t(hi)), __uint_as_float(uint32_t(hi >> 32)));
+}
+__device__ __forceinline__ void stWord(float4* p, float x, float y, float z, uint32_t tag) {
+  const unsigned long long lo = (unsigned long long)__float_as_uint(x) | ((unsigned long long)__float_as_uint(y) << 32);
+  const unsigned long long hi = (unsigned long long)__float_as_uint(z) | ((unsigned long long)tag << 32);
+  asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p), "l"(lo), "l"(hi) : "memory");
+}
+__device__ __forceinline__ uint32_t tagOf(float4 v) { return __float_as_uint(v.w); }
+// Uses the parts of a polled word that its reader has no need of, always false: with a part unused the
+// assembler narrows the access to several smaller ones, and a tag could arrive with an older value.
+__device__ __forceinline__ bool brokenWord(float4 v) { return (__float_as_uint(v.y) & __float_as_uint(v.z)) == 0xffffffffu; }
+
+// A body's four words: displacement | 2 vec r | rotation x y z | rotation w, r's w, a filler
+constexpr int BODY_WORDS = 4;
+__device__ __forceinline__ void stBody(const DWorld& w, uint32_t i, float3 dl, float4 dang, float4 q, uint32_t tag) {
+  float4* b = w.words + size_t(i) * BODY_WORDS;
+  stWord(b, dl.x, dl.y, dl.z, tag);
+  stWord(b + 1, dang.x, dang.y, dang.z, tag);
+  stWord(b + 2, q.x, q.y, q.z, tag);
+  stWord(b + 3, q.w, dang.w, dl.x, tag);
+}
+
+// Keeps a waiting lane's polls bounded: false past the clock budget, or once any wait of the launch
+// gave up.
+struct PollLimit {
+  long long t0 = 0;
+  uint32_t n = 0;
+  __device__ __forceinline__ bool again(const DWorld& w) {
+    if (n++ == 0u) {
+      t0 = clock64();
+      return true;
+    }
     if (n > 64u) __nanosleep(32);
-    if (ld_acquire_gpu(flag) >= need) return true;
     if ((n & 15u) == 0u) {
       if (ldv(&w.counters[C_ERROR]) & ERR_DEPENDENCY_TIMEOUT) return false;
       if (clock64() - t0 > BARRIER_CYCLES) {
@@ -736,7 +827,15 @@ __device__ inline bool waitDone(const DWorld& w, const uint32_t* flag, uint32_t 
         return false;
       }
     }
+    return true;
   }
+};
+// Waits until a body's joint count (published with release semantics) reaches `need`
+__device__ inline bool waitDone(const DWorld& w, const uint32_t* flag, uint32_t need) {
+  PollLimit limit;
+  while (ld_acquire_gpu(flag) < need)
+    if (!limit.again(w)) return false;
+  return true;
 }
 
 __device__ __forceinline__ void st_release_gpu(uint32_t* p, uint32_t v) {
@@ -784,42 +883,63 @@ __device__ __forceinline__ LaneJob laneJob(const DWorld& w, uint32_t c, uint32_t
   return J;
 }
 
-// The count a lane waits for before reading an incidence's partner (null: a static partner, no
-// wait). A partner of an earlier colour must have moved in this iteration: its pose is all this body
-// reads of it (their shared rows are this body's to update). One of a later colour must have finished
-// the previous iteration, pose and the rows it updates, these among them. A partner of the same colour
-// (only where the colour cap forced a clash) is not waited for within the iteration: the
-// colour-by-colour sweep runs such pairs side by side too.
-__device__ __forceinline__ const uint32_t* partnerFlag(const DWorld& w, uint2 inc, uint32_t it, uint32_t& need) {
-  need = 0u;
-  if (!(inc.y & PARTNER_DYNAMIC)) return nullptr;
-  const uint32_t partner = inc.y & PARTNER_MASK;
-  if (inc.y & PARTNER_EARLIER) {
-    need = it + 1u;
-    return w.poseDone + partner;
+// A body's state as the solve reads it, and its inertia, into its first lane's system: M (x - y) and
+// I qsub(q, y's rotation), both relative to x-: (dlin - ylin) and qsub(r, yang)
+__device__ __forceinline__ void addInertia(Acc& acc, const DWorld& w, uint32_t body, const Pose& own, float dt2) {
+  float m = w.size[body].w / dt2;
+  float3 I = f3(w.moment[body]) / dt2;
+  acc.v[0] = m;
+  acc.v[3] = m;
+  acc.v[5] = m;
+  acc.v[6] = I.x;
+  acc.v[9] = I.y;
+  acc.v[11] = I.z;
+  float3 rl = (own.dLin - f3(w.ylin[body])) * m;
+  float3 ra = I * qsub(relRot(own.dAng, own.rw), w.yang[body]);
+  acc.v[21] = rl.x;
+  acc.v[22] = rl.y;
+  acc.v[23] = rl.z;
+  acc.v[24] = ra.x;
+  acc.v[25] = ra.y;
+  acc.v[26] = ra.z;
+}
+// Sums the groups' systems: as many butterfly rounds as the warp's widest group needs
+__device__ __forceinline__ void sumGroup(Acc& acc, uint32_t L) {
+  const uint32_t Lmax = __reduce_max_sync(0xffffffffu, L);
+  for (uint32_t off = Lmax >> 1; off > 0; off >>= 1) {
+    const bool take = off < L;
+#pragma unroll
+    for (int k = 0; k < 27; k++) {
+      float o = __shfl_xor_sync(0xffffffffu, acc.v[k], off);
+      if (take) acc.v[k] += o;
+    }
   }
-  need = it;
-  return w.done + partner;
+}
+// The Newton step applied: the body's new displacement, dang word and rotation
+__device__ __forceinline__ void newPose(const Acc& acc, const Pose& own, float3& dl, float4& dw, float4& q) {
+  float3 dx, dth;
+  finishBody(acc, dx, dth);
+  dl = dl - dx;
+  const float4 r = qadd(relRot(own.dAng, own.rw), make_float3(-dth.x, -dth.y, -dth.z));
+  q = qnormalize4(qmul(r, own.q0));
+  dw = dangWord(r);
+}
+// The group's leader's new pose, to all its lanes
+__device__ __forceinline__ void sharePose(Pose& own, float3 dl, float3 da, float4 q, uint32_t leader) {
+  own.q = make_float4(__shfl_sync(0xffffffffu, q.x, leader), __shfl_sync(0xffffffffu, q.y, leader), __shfl_sync(0xffffffffu, q.z, leader),
+                      __shfl_sync(0xffffffffu, q.w, leader));
+  own.dLin = make_float3(__shfl_sync(0xffffffffu, dl.x, leader), __shfl_sync(0xffffffffu, dl.y, leader), __shfl_sync(0xffffffffu, dl.z, leader));
+  own.dAng = make_float3(__shfl_sync(0xffffffffu, da.x, leader), __shfl_sync(0xffffffffu, da.y, leader), __shfl_sync(0xffffffffu, da.z, leader));
 }
 
-// One 32-lane chunk: each group of lanes (one body) accumulates its rows, sums them by butterfly, its
-// first lane solves and writes the pose, and the lanes update the rows the body owns. With kWait the
-// chunk waits for the partner bodies it reads and afterwards publishes its bodies' iteration count;
-// false: a wait gave up (warp-uniform). With kWait the caller runs a chunk on the same warp in every
-// iteration, so the chunk's own bodies were last written by this warp (ordered by its __syncwarp)
-// and need no wait: their state is loaded first, alongside the first two rows' incidences, and only the
-// partners' counts are awaited (those of the first two rows polled together).
-template <bool kWait>
-__device__ __forceinline__ bool solveLanes(const DWorld& w, const StepParams& p, const LaneJob& J, uint32_t it) {
+// One 32-lane chunk at block scope: each group of lanes (one body) accumulates its rows, sums them by
+// butterfly, its first lane solves and writes the pose, and the lanes update the rows the body owns.
+__device__ __forceinline__ void solveLanes(const DWorld& w, const StepParams& p, const LaneJob& J) {
   const uint32_t lane = threadIdx.x & 31u;
   const float dt2 = p.dt * p.dt;
   const bool active = J.active;
   const uint32_t L = J.L, sub = J.sub, body = J.body, e1 = J.e1;
   const uint32_t leader = lane - sub;
-  // the incidence list is fixed for the step: the lane's first two rows are read before any wait
-  const uint32_t eB = J.e + L;
-  const uint2 inc0 = kWait && active && J.e < e1 ? w.incList[J.e] : make_uint2(0u, 0u);
-  const uint2 inc1 = kWait && active && eB < e1 ? w.incList[eB] : make_uint2(0u, 0u);
   Pose own;
   Acc acc;
   accZero(acc);
@@ -851,25 +971,8 @@ __device__ __forceinline__ bool solveLanes(const DWorld& w, const StepParams& p,
       acc.v[26] = ra.z;
     }
   }
-  if constexpr (kWait) {
-    bool ok = true;
-    uint32_t needA, needB;
-    const uint32_t* fA = active && J.e < e1 ? partnerFlag(w, inc0, it, needA) : nullptr;
-    const uint32_t* fB = active && eB < e1 ? partnerFlag(w, inc1, it, needB) : nullptr;
-    const uint32_t vA = fA ? ld_acquire_gpu(fA) : 0u;
-    const uint32_t vB = fB ? ld_acquire_gpu(fB) : 0u;
-    if (fA && vA < needA) ok = waitDone(w, fA, needA);
-    if (ok && fB && vB < needB) ok = waitDone(w, fB, needB);
-    if (active)
-      for (uint32_t e = eB + L; e < e1 && ok; e += L) {
-        uint32_t need;
-        const uint32_t* f = partnerFlag(w, w.incList[e], it, need);
-        if (f) ok = waitDone(w, f, need);
-      }
-    if (__any_sync(0xffffffffu, !ok)) return false;
-  }
   if (active)
-    for (uint32_t e = J.e; e < e1; e += L) accumulateIncidence(acc, w, p, kWait && e == J.e ? inc0 : kWait && e == eB ? inc1 : w.incList[e], body, own);
+    for (uint32_t e = J.e; e < e1; e += L) accumulateIncidence(acc, w, p, w.incList[e], body, own);
   // butterfly over the group: as many rounds as the warp's widest group needs
   const uint32_t Lmax = __reduce_max_sync(0xffffffffu, L);
   for (uint32_t off = Lmax >> 1; off > 0; off >>= 1) {
@@ -893,8 +996,6 @@ __device__ __forceinline__ bool solveLanes(const DWorld& w, const StepParams& p,
     w.rot[body] = q;
     w.dlin[body] = make_float4(dl.x, dl.y, dl.z, 0.0f);
     w.dang[body] = dw;
-    // the pose is final for this iteration: partners of later colours may read it now
-    if constexpr (kWait) st_release_gpu(w.poseDone + body, it + 1u);
   }
   own.q = make_float4(__shfl_sync(0xffffffffu, q.x, leader), __shfl_sync(0xffffffffu, q.y, leader), __shfl_sync(0xffffffffu, q.z, leader),
                       __shfl_sync(0xffffffffu, q.w, leader));
@@ -902,16 +1003,184 @@ __device__ __forceinline__ bool solveLanes(const DWorld& w, const StepParams& p,
   own.dAng = make_float3(__shfl_sync(0xffffffffu, da.x, leader), __shfl_sync(0xffffffffu, da.y, leader), __shfl_sync(0xffffffffu, da.z, leader));
   if (active) {
     for (uint32_t e = J.e; e < e1; e += L) {
-      const uint2 inc = kWait && e == J.e ? inc0 : w.incList[e];
+      const uint2 inc = w.incList[e];
       if (inc.x & OWNER_BIT) dualIncidence(w, p, inc, body, own);
     }
   }
-  if constexpr (kWait) {
-    // the group's writes (the leader's pose, every lane's rows) are ordered before the leader's
-    // release by the warp barrier, as the grid barrier orders a block's writes before its arrival
-    __syncwarp();
-    if (active && sub == 0) st_release_gpu(w.done + body, it + 1u);
+}
+
+// A contact row of the dataflow sweep as it is loaded: the parts fixed for the step, its two words and
+// its partner's four
+struct FlowRow {
+  float4 ra, rb, geo, pen, lam, b0, b1, b2, b3;
+  float2 c0t;
+};
+__device__ __forceinline__ void issueRow(const DWorld& w, const StepParams& p, uint2 inc, FlowRow& f) {
+  const uint32_t cs = (inc.x & ~OWNER_BIT) - p.nj;
+  const float4* pt = w.cPt[p.cur] + 4 * size_t(cs);
+  const float4* b = w.words + size_t(inc.y & PARTNER_MASK) * BODY_WORDS;
+  f.b0 = ldWord(b);
+  f.b1 = ldWord(b + 1);
+  f.b2 = ldWord(b + 2);
+  f.b3 = ldWord(b + 3);
+  f.pen = ldWord(pt + K_PEN);
+  f.lam = ldWord(pt + K_LAM);
+  f.ra = pt[K_RA];
+  f.rb = pt[K_RB];
+  f.c0t = w.c0t[cs];
+  f.geo = w.mGeo[p.cur][cs / MAX_CONTACTS];
+}
+// The tags a lane waits for. A dynamic partner of an earlier colour must have moved in this iteration;
+// one of a later colour, in the one before, and it also updates the shared rows, after the pose. A
+// static partner and the rows this body updates itself are always there. A partner of the same colour
+// (only where the colour cap forced a clash) is not waited for within the iteration: the
+// colour-by-colour sweep runs such pairs side by side too.
+__device__ __forceinline__ uint32_t needPose(uint32_t partnerWord, uint32_t it) {
+  return (partnerWord & PARTNER_DYNAMIC) ? ((partnerWord & PARTNER_EARLIER) ? it + 1u : it) : 0u;
+}
+__device__ __forceinline__ bool settleRow(const DWorld& w, const StepParams& p, uint2 inc, uint32_t it, FlowRow& f) {
+  const uint32_t need = needPose(inc.y, it), needRow = (inc.x & OWNER_BIT) ? 0u : it;
+  const float4* pt = w.cPt[p.cur] + 4 * size_t((inc.x & ~OWNER_BIT) - p.nj);
+  const float4* b = w.words + size_t(inc.y & PARTNER_MASK) * BODY_WORDS;
+  PollLimit limit;
+  for (;;) {
+    const bool m0 = tagOf(f.b0) < need, m1 = tagOf(f.b1) < need, m2 = tagOf(f.b2) < need, m3 = tagOf(f.b3) < need || brokenWord(f.b3);
+    const bool mp = tagOf(f.pen) < needRow, ml = tagOf(f.lam) < needRow;
+    if (!(m0 | m1 | m2 | m3 | mp | ml)) return true;
+    if (!limit.again(w)) return false;
+    if (m0) f.b0 = ldWord(b);
+    if (m1) f.b1 = ldWord(b + 1);
+    if (m2) f.b2 = ldWord(b + 2);
+    if (m3) f.b3 = ldWord(b + 3);
+    if (mp) f.pen = ldWord(pt + K_PEN);
+    if (ml) f.lam = ldWord(pt + K_LAM);
   }
+}
+__device__ __forceinline__ Pose wordPose(float4 b0, float4 b1, float4 b2, float4 b3) {
+  Pose P;
+  P.q = make_float4(b2.x, b2.y, b2.z, b3.x);
+  P.dLin = f3(b0);
+  P.dAng = f3(b1);
+  P.x0 = make_float3(0.0f, 0.0f, 0.0f);
+  P.q0 = P.q;
+  P.rw = b3.y;
+  return P;
+}
+__device__ __forceinline__ void flowPoint(const DWorld& w, uint2 inc, uint32_t body, const FlowRow& f, PointView& v) {
+  v.ra = f.ra;
+  v.rb = f.rb;
+  v.pen = make_float4(f.pen.x, f.pen.y, f.pen.z, f.c0t.x);
+  v.lam = make_float4(f.lam.x, f.lam.y, f.lam.z, f.c0t.y);
+  v.other = wordPose(f.b0, f.b1, f.b2, f.b3);
+  viewPoint(w, f.geo, body, inc.y & PARTNER_MASK, v);
+}
+// A joint's partner (its words polled) and, when the partner updates the joint, that update awaited
+constexpr uint32_t WORLD_PARTNER = 0x7fffffffu & PARTNER_MASK;  // a world joint's other end
+__device__ inline bool flowJoint(const DWorld& w, uint2 inc, uint32_t it, Pose& P) {
+  const uint32_t partner = inc.y & PARTNER_MASK;
+  if (partner == WORLD_PARTNER) return true;
+  const uint32_t need = needPose(inc.y, it);
+  const float4* b = w.words + size_t(partner) * BODY_WORDS;
+  float4 v[BODY_WORDS];
+  PollLimit limit;
+#pragma unroll
+  for (int k = 0; k < BODY_WORDS; k++) {
+    v[k] = ldWord(b + k);
+    while (tagOf(v[k]) < need || brokenWord(v[k])) {
+      if (!limit.again(w)) return false;
+      v[k] = ldWord(b + k);
+    }
+  }
+  P = wordPose(v[0], v[1], v[2], v[3]);
+  P.x0 = f3(w.ipos[partner]);
+  return (inc.x & OWNER_BIT) || it == 0u || waitDone(w, w.done + partner, it);
+}
+
+// One 32-lane chunk of the dataflow sweep, solveLanes with every word awaited (above) and written with
+// its tag. The caller runs a chunk on the same warp in every iteration, so a chunk's own bodies and rows
+// were last written by this warp and need no wait. False: a wait gave up (warp-uniform).
+__device__ __forceinline__ bool flowLanes(const DWorld& w, const StepParams& p, const LaneJob& J, uint32_t it) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const float dt2 = p.dt * p.dt;
+  const bool active = J.active, last = it + 1u == (uint32_t)p.iterations;
+  const uint32_t L = J.L, sub = J.sub, body = J.body, e1 = J.e1;
+  Pose own;
+  Acc acc;
+  accZero(acc);
+  bool ok = true, joints = false;
+  if (active) {
+    const float4* b = w.words + size_t(body) * BODY_WORDS;
+    own = wordPose(ldWord(b), ldWord(b + 1), ldWord(b + 2), ldWord(b + 3));
+    own.q0 = w.irot[body];
+    if (p.nj) own.x0 = f3(w.ipos[body]);
+    if (sub == 0) addInertia(acc, w, body, own, dt2);
+    for (uint32_t e = J.e; e < e1 && ok; e += L) {
+      const uint2 inc = w.incList[e];
+      if ((inc.x & ~OWNER_BIT) < p.nj) {
+        Pose P = own;
+        ok = flowJoint(w, inc, it, P);
+        if (ok) {
+          PosePair B{body, &own, &P};
+          addJoint(acc, w, inc.x & ~OWNER_BIT, p.alpha, body, B);
+        }
+        joints = joints || (inc.x & OWNER_BIT);
+        continue;
+      }
+      FlowRow f;
+      issueRow(w, p, inc, f);
+      ok = settleRow(w, p, inc, it, f);
+      if (ok) {
+        PointView v;
+        flowPoint(w, inc, body, f, v);
+        addView(acc, v, own, p.alpha);
+      }
+    }
+  }
+  if (__any_sync(0xffffffffu, !ok)) return false;
+  sumGroup(acc, L);
+  float3 dl = own.dLin, da = own.dAng;
+  float4 q = own.q;
+  if (active && sub == 0) {
+    float4 dw;
+    newPose(acc, own, dl, dw, q);
+    da = f3(dw);
+    stBody(w, body, dl, dw, q, it + 1u);
+  }
+  sharePose(own, dl, da, q, lane - sub);
+  if (active) {
+    for (uint32_t e = J.e; e < e1; e += L) {
+      const uint2 inc = w.incList[e];
+      if (!(inc.x & OWNER_BIT)) continue;
+      if ((inc.x & ~OWNER_BIT) < p.nj) {
+        Pose P = own;
+        if (flowJoint(w, inc, it, P)) {
+          PosePair B{body, &own, &P};
+          dualJoint(w, p, inc.x & ~OWNER_BIT, B);
+        }
+        continue;
+      }
+      // the partner's words are as they were read above: it moves again only after this row's tag
+      FlowRow f;
+      issueRow(w, p, inc, f);
+      PointView v;
+      flowPoint(w, inc, body, f, v);
+      float4 pen, lam;
+      uint32_t key;
+      dualView(v, own, p, pen, lam, key);
+      float4* pt = w.cPt[p.cur] + 4 * size_t((inc.x & ~OWNER_BIT) - p.nj);
+      if (key != __float_as_uint(v.ra.w)) pt[K_RA].w = __uint_as_float(key);
+      // the last iteration leaves the record as the contact layout has it, C0's parts in place of the tags
+      stWord(pt + K_PEN, pen.x, pen.y, pen.z, last ? __float_as_uint(pen.w) : it + 1u);
+      stWord(pt + K_LAM, lam.x, lam.y, lam.z, last ? __float_as_uint(lam.w) : it + 1u);
+    }
+  }
+  if (p.nj) {  // joints are updated in place, word by word: their readers wait for a count instead
+    const uint32_t mask = __ballot_sync(0xffffffffu, joints);
+    const uint32_t group = L >= 32u ? 0xffffffffu : ((1u << L) - 1u) << (lane - sub);
+    __syncwarp();
+    if (active && sub == 0 && (mask & group)) st_release_gpu(w.done + body, it + 1u);
+  }
+  __syncwarp();
   return true;
 }
 
@@ -1251,7 +1520,7 @@ __device__ void topologySolve(const DWorld& w, const StepParams& p, Team& team) 
     int a = info.y, b = info.z;
     if ((a >= 0 && !enabledBody(w, (uint32_t)a)) || !enabledBody(w, (uint32_t)b)) continue;
     float4 k[JOINT_VEC4];
-    loadJoint(w, j, k);
+    loadJoint<false>(w, j, k);
     Pose dummy;
     Bodies2 B{&w, 0xffffffffu, &dummy, true};
     float3 cl = jointLinC(k, a, b, B), ca = jointAngC(k, a, b, B);
@@ -1279,10 +1548,7 @@ __device__ void topologySolve(const DWorld& w, const StepParams& p, Team& team) 
   const float3 up = make_float3(p.upx, p.upy, p.upz);
   const uint32_t stepWord = ldv(&ctr[C_STEP]);  // steps since the world was made, from 1
   for (uint32_t i = tid; i < n; i += T) {
-    if constexpr (Team::kDataflow) {
-      w.done[i] = 0u;
-      w.poseDone[i] = 0u;
-    }
+    if constexpr (Team::kDataflow) w.done[i] = 0u;
     if (!enabledBody(w, i)) continue;
     float4 pos = w.pos[i], rot = w.rot[i], vel = w.vel[i];
     float3 av = f3(w.avel[i]);
@@ -1335,8 +1601,12 @@ __device__ void topologySolve(const DWorld& w, const StepParams& p, Team& team) 
     const float4 q = moved ? qnormalize4(qmul(r, rot)) : rot;
     w.pos[i] = make_float4(x.x, x.y, x.z, pos.w);
     w.rot[i] = q;
-    w.dlin[i] = make_float4(dl.x, dl.y, dl.z, 0.0f);
-    w.dang[i] = dangWord(r);
+    if constexpr (Team::kDataflow) {
+      stBody(w, i, dl, dangWord(r), q, 0u);
+    } else {
+      w.dlin[i] = make_float4(dl.x, dl.y, dl.z, 0.0f);
+      w.dang[i] = dangWord(r);
+    }
   }
   GSYNC
 
@@ -1395,14 +1665,14 @@ __device__ void topologySolve(const DWorld& w, const StepParams& p, Team& team) 
     for (uint32_t j = 0; j < items; j++) {
       const LaneJob J = jobFromEntry(next, nextActive);
       next = entryOf(j + 1u, nextActive);
-      if (!solveLanes<true>(w, p, J, j / mine)) break;
+      if (!flowLanes(w, p, J, j / mine)) break;
     }
     GSYNC
   } else {
     for (int it = 0; it < p.iterations; it++) {
       for (uint32_t c = 0; c < numColors; c++) {
         for (uint32_t base = warpGlobal * 32u; base < s_total[c]; base += nwarps * 32u)
-          solveLanes<false>(w, p, laneJob(w, c, base, s_lane, s_start, s_total), (uint32_t)it);
+          solveLanes(w, p, laneJob(w, c, base, s_lane, s_start, s_total));
         GSYNC
       }
     }
@@ -1415,13 +1685,23 @@ __device__ void topologySolve(const DWorld& w, const StepParams& p, Team& team) 
     float prevUp = dot3(f3(vel), up);
     if (w.size[i].w > 0.0f) {
       // x = x- + the displacement (the sweep keeps only the displacement, which partners read)
-      const float3 dl = f3(w.dlin[i]);
+      float3 dl, dang;
+      if constexpr (Team::kDataflow) {
+        const float4* b = w.words + size_t(i) * BODY_WORDS;
+        const float4 b2 = ldWord(b + 2);
+        dl = f3(ldWord(b));
+        dang = f3(ldWord(b + 1));
+        w.rot[i] = make_float4(b2.x, b2.y, b2.z, ldWord(b + 3).x);
+      } else {
+        dl = f3(w.dlin[i]);
+        dang = f3(w.dang[i]);
+      }
       const float3 x = f3(w.ipos[i]) + dl;
       w.pos[i] = make_float4(x.x, x.y, x.z, w.pos[i].w);
       // (x - x-) / dt and qsub(q, q-) / dt: the step's displacement and 2 vec(r)
       float3 v = dl / dt;
       w.vel[i] = make_float4(v.x, v.y, v.z, prevUp);
-      float3 av = f3(w.dang[i]) / dt;
+      float3 av = dang / dt;
       w.avel[i] = make_float4(av.x, av.y, av.z, w.avel[i].w);
     } else {
       w.vel[i] = make_float4(vel.x, vel.y, vel.z, prevUp);
@@ -1431,14 +1711,17 @@ __device__ void topologySolve(const DWorld& w, const StepParams& p, Team& team) 
 #undef GSYNC
 }
 
-__global__ void __launch_bounds__(SOLVE_THREADS, 2) k_topology_solve(DWorld w, StepParams p) {
+// Instantiated for one and for two blocks an SM: one gives every thread up to 255 registers, so that
+// the sweep's rows stay out of local memory, two twice the warps to hide each other's waits.
+template <int kBlocksPerSm>
+__global__ void __launch_bounds__(SOLVE_THREADS, kBlocksPerSm) k_topology_solve(DWorld w, StepParams p) {
   if (threadIdx.x == 0) s_epoch = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     g_clocks = w.clocks;
     w.clocks[0] = 1;
     w.clocks[1] = globaltimer();
   }
-  GridTeam team{w.barrier, w.counters};
+  GridTeam team{w.barrier, w.counters, p.laneBudget};
   topologySolve(w, p, team);
 }
 
@@ -1518,20 +1801,33 @@ cudaError_t launch_batch_solve(const BatchLaunch& b, int blocks, int worldThread
 int solve_grid_blocks(int device) {
   int sms = 0, perSm = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_topology_solve, SOLVE_THREADS, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_topology_solve<2>, SOLVE_THREADS, 0);
   if (perSm < 1) perSm = 1;
   return sms * perSm;
 }
 
-cudaError_t launch_topology_solve(const DWorld& w, const StepParams& p, int blocks, cudaStream_t s) {
+// The launch of a world of n bodies: `blocks` of them, or, for 0, by size. Up to SMALL_SOLVE bodies
+// the sweep is a chain of colours, each waiting on the one before with few chunks a warp: one block an
+// SM with all its registers is faster (3001 bodies: solve 0.203 ms against 0.233), and fewer blocks
+// meet sooner at the barriers between the topology's phases, so long as a colour's rows still get a
+// lane each (a block for 16 bodies; 48 boxes: a step of 82 us against about 150 with every block). Past
+// it the chunks outnumber the warps and two blocks an SM win (20000 bodies: 0.369 ms against 0.398;
+// 100000: 1.30 against 1.60).
+constexpr uint32_t SMALL_SOLVE = 8192;
+cudaError_t launch_topology_solve(const DWorld& w, const StepParams& p, int blocks, int maxBlocks, int sms, cudaStream_t s) {
+  const bool one = p.n <= SMALL_SOLVE && blocks <= sms;
+  StepParams pc = p;
+  // the lane classes, and with them the order in which a body's rows are summed, do not follow the size
+  pc.laneBudget = blocks <= 0 ? uint32_t(maxBlocks) * SOLVE_THREADS : 0u;
+  if (blocks <= 0) blocks = one ? std::min<int>(sms, std::max<int>(1, int(p.n + 15u) / 16)) : maxBlocks;
   cudaMemsetAsync(w.barrier, 0, 2 * sizeof(uint32_t), s);
   cudaMemsetAsync(w.adjStart, 0, (size_t(p.n) + 1) * sizeof(uint32_t), s);
   cudaMemsetAsync(w.adjFill, 0, (size_t(p.n) + 1) * sizeof(uint32_t), s);
   cudaMemsetAsync(w.bucket, 0, BUCKET_WORDS * sizeof(uint32_t), s);
   DWorld wc = w;
-  StepParams pc = p;
   void* args[] = {&wc, &pc};
-  return cudaLaunchCooperativeKernel((const void*)k_topology_solve, dim3(blocks), dim3(SOLVE_THREADS), args, 0, s);
+  const void* kernel = one ? (const void*)k_topology_solve<1> : (const void*)k_topology_solve<2>;
+  return cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(SOLVE_THREADS), args, 0, s);
 }
 
 }  // namespace avbd
