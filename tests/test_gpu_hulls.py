@@ -48,6 +48,50 @@ def test_hull_narrowphase_known_answers(cuda_lib):
     assert pairs64 >= 190
 
 
+@pytest.mark.parametrize('sides', [3, 5, 16, 31])
+def test_many_sided_faces_clip_as_the_oracle_clips(cuda_lib, sides):
+    """Cones resting base to base, turned against each other, and a cone's base on a box: the clipped
+    polygons have up to twice the base's corners (62, past a warp's lanes). Contacts bit for bit the f32
+    restatement's."""
+    from avbd_b200.hulls import build_hull
+    from avbd_b200.scenes import Scene
+    rng = np.random.default_rng(sides)
+    ring = np.arange(sides) * 2.0 * np.pi / sides
+    shape = build_hull(np.concatenate([np.stack([0.8 * np.cos(ring), 0.8 * np.sin(ring), 0 * ring], 1), [[0.0, 0.0, 0.7]]]).reshape(-1))
+    s = Scene('cones')
+    s.params.gravity = 0.0
+    s.params.iterations = 0
+    at = s.add_hull_shape(shape)
+    low = float(shape.vertices[:, 2].min())
+    pairs = 24
+    for k in range(pairs):
+        x = np.array([5.0 * k, 0.0, 0.0])
+        tilt = rng.normal(0, 2e-3, 2)
+        yaw = rng.uniform(0, np.pi)
+        q = np.array([tilt[0], tilt[1], np.sin(yaw / 2), np.cos(yaw / 2)])
+        if k % 3 == 2:
+            s.box([1.0, 1.1, 0.5], 1.0, 0.5, (x - [0, 0, 0.25]).tolist())
+        else:  # upside down: its base up
+            s.hull(shape, 1.0, 0.5, (x + [0, 0, low]).tolist(), [1.0, 0.0, 0.0, 0.0], offset=at)
+        s.hull(shape, 1.0, 0.5, (x + [*rng.uniform(-0.3, 0.3, 2), -low - 0.01]).tolist(), (q / np.linalg.norm(q)).tolist(), offset=at)
+    w = avbd_b200.CudaSolver3D(s)
+    w.step()
+    contacts = w.read_contact_list()
+    o32 = Oracle(s, fp32=True)
+    total = 0
+    for p in range(pairs):
+        a, b = 2 * p + 1, 2 * p
+        mine = [x for x in contacts if x['a'] == a and x['b'] == b]
+        exact, _ = o32.narrowphase(a, b)
+        assert len(mine) == len(exact), f'pair {p}: {len(mine)} contacts vs {len(exact)}'
+        total += len(exact)
+        for x, (f, ra, rb) in zip(mine, exact):
+            assert x['feature'] == f
+            assert np.array_equal(x['rA'].astype(np.float32), ra.astype(np.float32)) and np.array_equal(x['rB'].astype(np.float32), rb.astype(np.float32))
+    assert total >= 3 * pairs and len(contacts) == total
+    w.destroy()
+
+
 def test_hull_pile_coloured_step_matches_fp64(cuda_lib):
     """A pile of hulls, boxes and spheres (coloured mode): from the oracle's state after 70 GPU-mode
     steps, one GPU step against one FP64 step with the oracle's colours; poses within 1e-5."""
