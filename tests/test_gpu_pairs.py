@@ -1,0 +1,60 @@
+"""The step's pair walk and the tables it shares between steps: pair sets against the no-allocation
+broadphase (one thread a body) and the oracle's grid, over several steps."""
+
+import numpy as np
+import pytest
+
+import avbd_b200
+from avbd_b200.scenes import Scene, drop_pile
+from oracle import Oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _pairs(a):
+    return {(int(x), int(y)) for x, y in a}
+
+
+@pytest.mark.parametrize('n', [1, 7, 15, 257, 4000])
+def test_pairs_follow_the_bodies_over_steps(cuda_lib, n):
+    """Boxes and spheres with large bodies among them, fixed and moving, some disabled: each step's pairs
+    are those of the poses it starts from."""
+    scene = drop_pile(n, seed=n, spacing=1.25, layers=3)
+    rng = np.random.default_rng(n)
+    if n >= 257:
+        for k in range(4):  # large: two fixed slabs, two moving ones
+            scene.box([9.0, 9.0, 0.5], 1.0 if k % 2 else 0, 0.5, [*rng.uniform(-6, 6, 2), 2.5 * k])
+    w = avbd_b200.CudaSolver3D(scene)
+    off = rng.choice(np.arange(1, n + 1), n // 20, replace=False) if n >= 257 else []
+    for i in off:
+        w.set_lifecycle(int(i), 2)
+    for step in range(6):
+        before = w.read_bodies()
+        want = _pairs(avbd_b200.find_pairs_noalloc(before))
+        w.step()
+        got = w.read_pairs()
+        assert len(got) == len(_pairs(got)), 'a pair twice'
+        assert _pairs(got) == want, f'step {step}'
+        w.step(3)
+    assert w.read_counters()['error'] == 0
+    w.destroy()
+
+
+@pytest.mark.parametrize('n', [32766, 32767, 32768])
+def test_pairs_on_both_sides_of_the_walks_widths(cuda_lib, n):
+    """With the ground 32767, 32768 and 32769 bodies: sixteen lanes a body up to 32768, four past it."""
+    scene = drop_pile(n, seed=3, spacing=1.3, layers=10)
+    w = avbd_b200.CudaSolver3D(scene)
+    o = Oracle(scene, fp32=True)
+    want = _pairs(o.pairs())
+    w.step()
+    assert _pairs(w.read_pairs()) == want and len(want) > n // 2
+    w.destroy()
+
+
+def test_a_world_without_bodies_steps(cuda_lib):
+    w = avbd_b200.CudaSolver3D(Scene('empty'), body_capacity=8)
+    w.step(3)
+    c = w.read_counters()
+    assert c['steps'] == 3 and c['pairs'] == 0 and c['error'] == 0
+    w.destroy()

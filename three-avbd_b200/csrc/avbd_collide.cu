@@ -1,6 +1,5 @@
 // Collision phase of the B200 AVBD step: last step's pairs into the warm-start hash, cell keys,
-// a counting sort of the bodies on their cell hash (a one-digit radix sort, stable by body index),
-// cell ranges, pair emission, and the narrowphase.
+// a counting sort of the bodies on their cell hash, pair emission, and the narrowphase.
 //
 // This file is compiled with --fmad=false: every product and sum is rounded on its own, in the
 // operation order of the reference's WGSL (src/avbd3d/gpu/wgsl-collision.ts), so the pair tests
@@ -36,8 +35,8 @@ __device__ __forceinline__ unsigned long long gtimer() {
   return t;
 }
 
-__global__ void k_begin(DWorld w, StepParams p) {
-  w.clocks[CLOCK_T0] = gtimer();
+// Last step's counters to this step's start (one thread)
+__device__ void rotateCounters(const DWorld& w, const StepParams& p) {
   uint32_t* c = w.counters;
   uint32_t pairs = c[C_PAIRS];
   c[C_PREV_PAIRS] = pairs < p.pairCap ? pairs : p.pairCap;
@@ -53,21 +52,22 @@ __global__ void k_begin(DWorld w, StepParams p) {
   c[C_HULL_PAIRS] = 0;
   for (int k = 0; k < 2 * MAX_ROUND_PAIRS + 2; k++) c[C_PENDING + k] = 0;
 }
+__global__ void k_begin(DWorld w, StepParams p) {
+  w.clocks[CLOCK_T0] = gtimer();
+  rotateCounters(w, p);
+}
 
 // --- last step's pairs into the hash table (wgsl-collision.ts:354-368), compare-and-swap probing ---
-__global__ void k_hash_insert(DWorld w, StepParams p) {
-  const int prev = 1 - p.cur;
-  const uint32_t count = w.counters[C_PREV_PAIRS];
-  for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < count; m += gridDim.x * blockDim.x) {
-    uint4 ids = w.mIds[prev][m];
-    if ((ids.w & 15u) == 0u) continue;
-    // Rewritten slots have no contact history
-    if (w.ipos[ids.x].w != 0.0f || w.ipos[ids.y].w != 0.0f) continue;
-    uint32_t h = pairHash(ids.x, ids.y) & p.hashMask;
-    for (uint32_t probe = 0; probe <= p.hashMask; probe++) {
-      if (atomicCAS(&w.hash[h], 0u, m + 1u) == 0u) break;
-      h = (h + 1u) & p.hashMask;
-    }
+// The table is empty here: the solve of the step before clears it, once the narrowphase is past it.
+__device__ __forceinline__ void hashInsert(const DWorld& w, const StepParams& p, uint32_t m) {
+  uint4 ids = w.mIds[1 - p.cur][m];
+  if ((ids.w & 15u) == 0u) return;
+  // Rewritten slots have no contact history
+  if (w.ipos[ids.x].w != 0.0f || w.ipos[ids.y].w != 0.0f) return;
+  uint32_t h = pairHash(ids.x, ids.y) & p.hashMask;
+  for (uint32_t probe = 0; probe <= p.hashMask; probe++) {
+    if (atomicCAS(&w.hash[h], 0u, m + 1u) == 0u) break;
+    h = (h + 1u) & p.hashMask;
   }
 }
 
@@ -82,6 +82,16 @@ __device__ inline int hashFind(const DWorld& w, const StepParams& p, uint32_t a,
     h = (h + 1u) & p.hashMask;
   }
   return -1;
+}
+
+// Clears what the solve starts from empty (degrees and fill cursors, the buckets, the grid barrier),
+// and the cell table, whose last reader was the pair walk, for the next step
+__device__ __forceinline__ void clearTables(const DWorld& w, const StepParams& p) {
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x;
+  for (uint32_t i = tid; i <= p.n; i += T) w.adjStart[i] = w.adjFill[i] = 0u;
+  for (uint32_t i = tid; i < (uint32_t)BUCKET_WORDS; i += T) w.bucket[i] = 0u;
+  for (uint32_t i = tid; i <= p.tableMask; i += T) w.cellStart[i] = 0u;
+  if (tid < 2u) w.barrier[tid] = 0u;
 }
 
 // --- contact reuse (wgsl-collision.ts:20-44, 706-762) -------------------------------------------------
@@ -193,6 +203,7 @@ __device__ inline bool reusePair(const DWorld& w, const StepParams& p, uint32_t 
 // reuseManifolds (wgsl-collision.ts:755-762): every pair slot of last step kept in the same slot,
 // its manifold copied; the step detects no pair
 __global__ void k_reuse_manifolds(DWorld w, StepParams p) {
+  clearTables(w, p);
   const uint32_t total = w.counters[C_PREV_PAIRS];
   const int prev = 1 - p.cur;
   if (blockIdx.x == 0 && threadIdx.x == 0) w.counters[C_PAIRS] = total;
@@ -215,107 +226,82 @@ __device__ inline uint32_t cellHash(int4 c, uint32_t mask) {
   return (((uint32_t)c.x * 73856093u) ^ ((uint32_t)c.y * 19349663u) ^ ((uint32_t)c.z * 83492791u)) & mask;
 }
 
-__global__ void k_cell_keys(DWorld w, StepParams p) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= p.n) return;
-  bool small = enabled(w, i) && w.moment[i].w <= p.largeThreshold;
-  int4 c = cellOf(f3(w.pos[i]), p.cellSize);
-  w.cell[i] = c;
-  w.keyA[i] = small ? cellHash(c, p.tableMask) : p.tableMask + 1u;  // large and disabled bodies sort last
-  w.valA[i] = i;
-}
-
 // --- counting sort of bodies by cell hash (a single radix pass on the whole key) -------------------
-// Count (each body keeps its rank in its bucket), exclusive scan of the bucket counts, scatter. The
-// order of bodies within a bucket follows the atomics and changes nothing downstream: pairs are a
-// set, and every body sums its rows in a sorted order of its own.
-__global__ void k_bucket_count(const uint32_t* keys, uint32_t n, uint32_t* count, uint32_t* rank, uint32_t sentinel) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint32_t k = keys[i];
-  rank[i] = k == sentinel ? 0u : atomicAdd(&count[k], 1u);
+// Count (each body keeps its rank in its bucket), a place for every bucket, scatter. Neither the order
+// of the buckets nor that of the bodies in one changes anything downstream: pairs are a set, and every
+// body sums its rows in a sorted order of its own. So a bucket takes its place from one counter, a block
+// of buckets at a time, and no scan over the table is needed.
+//
+// A step is a chain of dependent launches, 2 to 4 us each before they do any work: it took eighteen
+// (clears, a copy and three scan kernels among them), 48 bodies spending 74 us on collision, now 35. What
+// can be done together is: last step's pairs into the hash, the bodies' cells and counts and the reuse
+// reference poses, here; the tables that the next launches want empty are cleared by the launches that
+// read them last (k_narrowphase, the solve).
+__global__ void __launch_bounds__(256) k_prepare(DWorld w, StepParams p) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) w.clocks[CLOCK_T0] = gtimer();
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x;
+  const uint32_t prevPairs = min(w.counters[C_PAIRS], p.pairCap);  // k_cell_starts moves the counters on
+  for (uint32_t m = tid; m < prevPairs; m += T) hashInsert(w, p, m);
+  for (uint32_t i = tid; i < p.n; i += T) {
+    const bool on = enabled(w, i), small = on && w.moment[i].w <= p.largeThreshold;
+    const int4 c = cellOf(f3(w.pos[i]), p.cellSize);
+    w.cell[i] = c;
+    const uint32_t k = small ? cellHash(c, p.tableMask) : p.tableMask + 1u;  // large and disabled bodies are in no cell
+    w.keyA[i] = k;
+    if (small) w.valA[i] = atomicAdd(&w.cellStart[k], 1u);
+    if (on && (p.flags & FLAG_REUSE_CONTACTS)) updateRef(w, i, w.counters[C_STEP] + 1u);
+  }
 }
 
-// Exclusive scan, three kernels: block tiles of 4096 (totals out), the totals, the tiles' offsets.
-constexpr int SCAN_THREADS = 1024, SCAN_ITEMS = 4, SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
-__device__ uint32_t block_exclusive_scan_1024(uint32_t v, uint32_t* warpSums) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t x = v;
+// Every bucket's place: a block adds up its buckets' counts and takes a run of slots for them
+constexpr uint32_t STARTS_THREADS = 256, STARTS_ITEMS = 4;
+__global__ void __launch_bounds__(STARTS_THREADS) k_cell_starts(DWorld w, StepParams p) {
+  __shared__ uint32_t s_warp[STARTS_THREADS / 32], s_base;
+  if (blockIdx.x == 0 && threadIdx.x == 0) rotateCounters(w, p);
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t base = (blockIdx.x * STARTS_THREADS + threadIdx.x) * STARTS_ITEMS, len = p.tableMask + 1u;
+  uint32_t v[STARTS_ITEMS], sum = 0;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  if (lane == 31) warpSums[warp] = x;
-  __syncthreads();
-  if (warp == 0) {
-    uint32_t t = warpSums[lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
-      if (lane >= o) t += y;
-    }
-    warpSums[lane] = t;
-  }
-  __syncthreads();
-  uint32_t r = x - v + (warp > 0 ? warpSums[warp - 1] : 0u);
-  __syncthreads();
-  return r;
-}
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_tiles(uint32_t* data, uint32_t len, uint32_t* totals) {
-  __shared__ uint32_t warpSums[32];
-  uint32_t base = blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_ITEMS;
-  uint32_t v[SCAN_ITEMS], sum = 0;
-#pragma unroll
-  for (int k = 0; k < SCAN_ITEMS; k++) {
-    v[k] = base + k < len ? data[base + k] : 0u;
+  for (uint32_t k = 0; k < STARTS_ITEMS; k++) {
+    v[k] = base + k < len ? w.cellStart[base + k] : 0u;
     sum += v[k];
   }
-  uint32_t run = block_exclusive_scan_1024(sum, warpSums);
+  uint32_t x = sum;
 #pragma unroll
-  for (int k = 0; k < SCAN_ITEMS; k++) {
-    if (base + k < len) data[base + k] = run;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= (uint32_t)o) x += y;
+  }
+  if (lane == 31u) s_warp[warp] = x;
+  __syncthreads();
+  uint32_t before = 0, total = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < STARTS_THREADS / 32; k++) {
+    if (k < warp) before += s_warp[k];
+    total += s_warp[k];
+  }
+  if (threadIdx.x == 0) s_base = total ? atomicAdd(&w.counters[C_CELLS], total) : 0u;
+  __syncthreads();
+  uint32_t run = s_base + before + x - sum;
+#pragma unroll
+  for (uint32_t k = 0; k < STARTS_ITEMS; k++) {
+    if (base + k < len) {
+      w.cellStart[base + k] = run;
+      w.cellEnd[base + k] = run + v[k];
+    }
     run += v[k];
   }
-  if (threadIdx.x == SCAN_THREADS - 1) totals[blockIdx.x] = run;
-}
-__global__ void __launch_bounds__(1024) k_scan_single(uint32_t* data, uint32_t len) {
-  __shared__ uint32_t warpSums[32];
-  __shared__ uint32_t carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (uint32_t base = 0; base < len; base += 1024) {
-    uint32_t i = base + threadIdx.x;
-    uint32_t v = i < len ? data[i] : 0u;
-    uint32_t ex = block_exclusive_scan_1024(v, warpSums) + carry;
-    if (i < len) data[i] = ex;
-    __syncthreads();
-    if (threadIdx.x == 1023) carry = ex + v;
-    __syncthreads();
-  }
-}
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_add(uint32_t* data, uint32_t len, const uint32_t* totals) {
-  uint32_t add = totals[blockIdx.x];
-  uint32_t base = blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_ITEMS;
-#pragma unroll
-  for (int k = 0; k < SCAN_ITEMS; k++)
-    if (base + k < len) data[base + k] += add;
-}
-
-// cellEnd held the counts: make it start + count
-__global__ void k_bucket_finish(const uint32_t* start, uint32_t* end, uint32_t len) {
-  uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
-  if (h < len) end[h] += start[h];
 }
 
 // Bodies into bucket order, with each sorted slot's candidate record (position and radius, exact cell
 // and body with its dynamic bit) so a cell walk reads contiguous memory.
 __global__ void k_bucket_scatter(DWorld w, uint32_t n, uint32_t sentinel) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) w.counters[C_CELLS] = 0u;  // for the next step
   if (i >= n) return;
   uint32_t k = w.keyA[i];
   if (k == sentinel) return;
-  uint32_t slot = w.cellStart[k] + w.valB[i];
+  uint32_t slot = w.cellStart[k] + w.valA[i];
   float4 pi = w.pos[i];
   w.sortedPR[slot] = make_float4(pi.x, pi.y, pi.z, w.moment[i].w);
   int4 c = w.cell[i];
@@ -507,10 +493,15 @@ __device__ inline void largeAgainstLarge(const DWorld& w, const StepParams& p, c
   }
 }
 
-// One thread per body walks its cells with the cheap tests (cell, sphere, AABB); the candidates
-// that pass go to a per-warp queue in shared memory, and whenever it holds a warp's worth, the warp
-// takes the full test (the prober's view, the face separation, the no-collide list) one candidate a
-// lane, so that the long test runs on full warps instead of on the few lanes whose walk found one.
+// kLanes lanes a body walk its cells side by side with the cheap tests (cell, sphere, AABB), and the
+// large bodies after them; the candidates that pass go to a per-warp queue in shared memory, and
+// whenever it holds a warp's worth, the warp takes the full test (the prober's view, the face
+// separation, the no-collide list) one candidate a lane, so that the long test runs on full warps
+// instead of on the few lanes whose walk found one. The walk is bound by its dependent loads (bucket,
+// cell, position, AABB): one lane a body makes fifteen such chains one after another, sixteen lanes make
+// one each but all compute the body's AABB. Collision phase at 1, 4 and 16 lanes: 48 bodies 55, 39 and
+// 35 us; 3001: 127, 67, 47; 20000: 170, 96, 87; 100000: 310, 251, 291.
+constexpr uint32_t WALK_WIDE = 32768;  // bodies up to which sixteen lanes walk, four past it
 constexpr uint32_t PAIR_WALK_THREADS = 128, PAIR_QUEUE = 64;
 __device__ __forceinline__ void testCandidate(const DWorld& w, const StepParams& p, uint2 e) {
   const uint32_t pr = proberOf(w, p, e.x, e.y);
@@ -526,40 +517,52 @@ __device__ __forceinline__ void drainQueue(const DWorld& w, const StepParams& p,
   count -= take;
   if (lane < take) testCandidate(w, p, e);
 }
+constexpr uint32_t WALK_LARGE = 14;  // the place after the cells: the large bodies
+template <uint32_t kLanes>
 __global__ void __launch_bounds__(PAIR_WALK_THREADS) k_find_pairs(DWorld w, StepParams p) {
   __shared__ uint2 s_queue[PAIR_WALK_THREADS / 32][PAIR_QUEUE];
   const uint32_t lane = threadIdx.x & 31u;
   uint2* Q = s_queue[threadIdx.x >> 5];
   uint32_t count = 0;  // the warp's queue length (the same in every lane)
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
   const bool on = i < p.n && enabled(w, i);
   const bool dyn = on && w.size[i].w > 0.0f;
   const bool small = on && w.moment[i].w <= p.largeThreshold;
   float3 pos = make_float3(0.0f, 0.0f, 0.0f), aabb = pos;
   float radius = 0.0f;
-  int4 c = make_int4(0, 0, 0, 0);
+  int4 own = make_int4(0, 0, 0, 0);
   if (small) {
     pos = f3(w.pos[i]);
     radius = w.moment[i].w;
     aabb = aabbOf(w, i);
-    c = w.cell[i];
+    own = w.cell[i];
   }
 #pragma unroll 1
-  for (int o = 0; o < 14; o++) {
-    // offset o = 0: the own cell; 1..13: (dx, dy, dz) > 0 in (z, y, x) order
-    const int q = o == 0 ? 13 : 13 + o;
-    const int4 cc = make_int4(c.x + q % 3 - 1, c.y + (q / 3) % 3 - 1, c.z + q / 9 - 1, 0);
+  for (uint32_t o = lane % kLanes; o - lane % kLanes <= WALK_LARGE; o += kLanes) {
+    int4 cc = make_int4(0, 0, 0, 0);
     uint32_t k = 0, end = 0;
-    if (small) {
+    if (small && o < WALK_LARGE) {
+      // offset o = 0: the own cell; 1..13: (dx, dy, dz) > 0 in (z, y, x) order
+      const int q = o == 0u ? 13 : 13 + int(o);
+      cc = make_int4(own.x + q % 3 - 1, own.y + (q / 3) % 3 - 1, own.z + q / 9 - 1, 0);
       const uint32_t h = cellHash(cc, p.tableMask);
       k = w.cellStart[h];
       end = w.cellEnd[h];
+    } else if (o == WALK_LARGE && ((small && (dyn || p.anyDynamicLarge)) || (!small && dyn))) {
+      end = p.nLarge;
     }
     auto candidate = [&](uint32_t kk, uint32_t& jj) -> bool {
+      if (o == WALK_LARGE) {
+        // a small body against the large list, or a large dynamic body against it (each pair of large
+        // bodies once)
+        jj = w.large[kk];
+        if (!small) return jj != i && !(jj < i && w.size[jj].w > 0.0f);
+        return dyn || (enabled(w, jj) && w.size[jj].w > 0.0f);
+      }
       const int4 cj = w.sortedCell[kk];
       jj = (uint32_t)cj.w & 0x7fffffffu;
       const bool dj = ((uint32_t)cj.w & 0x80000000u) != 0u;
-      if ((o == 0 && jj >= i) || !(dyn || dj) || cj.x != cc.x || cj.y != cc.y || cj.z != cc.z) return false;
+      if ((o == 0u && jj >= i) || !(dyn || dj) || cj.x != cc.x || cj.y != cc.y || cj.z != cc.z) return false;
       const float4 pr = w.sortedPR[kk];
       const float3 d = pos - make_float3(pr.x, pr.y, pr.z);
       const float r = radius + pr.w;
@@ -567,30 +570,20 @@ __global__ void __launch_bounds__(PAIR_WALK_THREADS) k_find_pairs(DWorld w, Step
       const float4 ab = w.sortedAabb[kk];      // and the AABB test (its sums commute)
       return !(fabsf(d.x) > aabb.x + ab.x + 1e-4f || fabsf(d.y) > aabb.y + ab.y + 1e-4f || fabsf(d.z) > aabb.z + ab.z + 1e-4f);
     };
-    auto enqueue = [&](bool push, uint32_t jj) {
+    while (__any_sync(0xffffffffu, k < end)) {
+      uint32_t j = 0;
+      const bool push = k < end && candidate(k, j);
+      k++;
       const uint32_t m = __ballot_sync(0xffffffffu, push);
       if (m) {
-        if (push) Q[count + __popc(m & ((1u << lane) - 1u))] = make_uint2(i, jj);
+        if (push) Q[count + __popc(m & ((1u << lane) - 1u))] = make_uint2(i, j);
         count += __popc(m);
         __syncwarp();
         if (count >= 32u) drainQueue(w, p, Q, count, lane);
       }
-    };
-    while (__any_sync(0xffffffffu, k < end)) {
-      uint32_t j0 = 0, j1 = 0;
-      const bool p0 = k < end && candidate(k, j0);
-      const bool p1 = k + 1 < end && candidate(k + 1, j1);
-      k += 2;
-      enqueue(p0, j0);
-      enqueue(p1, j1);
     }
   }
   while (count > 0u) drainQueue(w, p, Q, count, lane);
-  if (small) {
-    smallAgainstLarge(w, p, probeOf(w, i), dyn);
-  } else if (dyn) {
-    largeAgainstLarge(w, p, probeOf(w, i));
-  }
 }
 
 // --- narrowphase: box SAT + clipping (wgsl-collision.ts:385-599, ref/collide.ts) ---------------------
@@ -1685,6 +1678,7 @@ __global__ void __launch_bounds__(HULL_THREADS) k_hull_narrowphase(DWorld w, Ste
 }
 
 __global__ void __launch_bounds__(128) k_narrowphase(DWorld w, StepParams p) {
+  clearTables(w, p);
   uint32_t total = w.counters[C_PAIRS];
   if (total > p.pairCap) total = p.pairCap;
   for (uint32_t pi = blockIdx.x * blockDim.x + threadIdx.x; pi < total; pi += gridDim.x * blockDim.x) narrowPair<true>(w, p, pi);
@@ -1802,36 +1796,28 @@ void launch_step_stats(const DWorld& w, uint32_t launches, cudaStream_t s) { k_s
 // Host: the collision phase, enqueued on `s`. Returns the number of kernels it launched.
 uint32_t launch_collision(const DWorld& w, const StepParams& p, uint32_t tableSize, bool reuseManifolds, cudaStream_t s) {
   const uint32_t n = p.n;
-  k_begin<<<1, 1, 0, s>>>(w, p);
-  uint32_t launches = 1;
-  if ((p.flags & FLAG_REUSE_CONTACTS) && n > 0) {
-    k_update_refs<<<grid_for(n, 256), 256, 0, s>>>(w, p);
-    launches++;
-  }
+  // grid-stride kernels over device-side counts: no more blocks than a small world has work for
+  const uint32_t gs = std::min<uint32_t>(GS_BLOCKS, 1u + n / 16u);
   if (reuseManifolds) {
-    k_reuse_manifolds<<<GS_BLOCKS, 128, 0, s>>>(w, p);
-    return launches + 1;
+    k_begin<<<1, 1, 0, s>>>(w, p);
+    uint32_t launches = 2;
+    if ((p.flags & FLAG_REUSE_CONTACTS) && n > 0) {
+      k_update_refs<<<grid_for(n, 256), 256, 0, s>>>(w, p);
+      launches++;
+    }
+    k_reuse_manifolds<<<gs, 128, 0, s>>>(w, p);
+    return launches;
   }
-  launches += 2;  // hash insert, narrowphase
-  cudaMemsetAsync(w.hash, 0, (size_t(p.hashMask) + 1) * 4, s);
-  k_hash_insert<<<GS_BLOCKS, 256, 0, s>>>(w, p);
+  k_prepare<<<std::min<uint32_t>(GS_BLOCKS, 1u + n / 64u), 256, 0, s>>>(w, p);
+  k_cell_starts<<<grid_for(tableSize, STARTS_THREADS * STARTS_ITEMS), STARTS_THREADS, 0, s>>>(w, p);
+  uint32_t launches = 3;
   if (n > 0) {
-    const uint32_t sentinel = p.tableMask + 1u;
-    cudaMemsetAsync(w.cellStart, 0, size_t(tableSize) * 4, s);
-    k_cell_keys<<<grid_for(n, 256), 256, 0, s>>>(w, p);
-    k_bucket_count<<<grid_for(n, 256), 256, 0, s>>>(w.keyA, n, w.cellStart, w.valB, sentinel);
-    // cellEnd = counts before the scan turns them into starts
-    cudaMemcpyAsync(w.cellEnd, w.cellStart, size_t(tableSize) * 4, cudaMemcpyDeviceToDevice, s);
-    uint32_t tiles = grid_for(tableSize, SCAN_TILE);
-    k_scan_tiles<<<tiles, SCAN_THREADS, 0, s>>>(w.cellStart, tableSize, w.radixHist);
-    k_scan_single<<<1, 1024, 0, s>>>(w.radixHist, tiles);
-    k_scan_add<<<tiles, SCAN_THREADS, 0, s>>>(w.cellStart, tableSize, w.radixHist);
-    k_bucket_finish<<<grid_for(tableSize, 256), 256, 0, s>>>(w.cellStart, w.cellEnd, tableSize);
-    k_bucket_scatter<<<grid_for(n, 256), 256, 0, s>>>(w, n, sentinel);
-    k_find_pairs<<<grid_for(n, PAIR_WALK_THREADS), PAIR_WALK_THREADS, 0, s>>>(w, p);
-    launches += 8;
+    k_bucket_scatter<<<grid_for(n, 128), 128, 0, s>>>(w, n, p.tableMask + 1u);
+    if (n <= WALK_WIDE) k_find_pairs<16><<<grid_for(n, PAIR_WALK_THREADS / 16), PAIR_WALK_THREADS, 0, s>>>(w, p);
+    else k_find_pairs<4><<<grid_for(n, PAIR_WALK_THREADS / 4), PAIR_WALK_THREADS, 0, s>>>(w, p);
+    launches += 2;
   }
-  k_narrowphase<<<GS_BLOCKS, 128, 0, s>>>(w, p);
+  k_narrowphase<<<gs, 128, 0, s>>>(w, p);
   if (w.hulls) {
     k_hull_narrowphase<<<std::min<uint32_t>(2u * GS_BLOCKS, 1u + n / 4u), HULL_THREADS, 0, s>>>(w, p);
     launches++;

@@ -49,6 +49,7 @@ constexpr int MAX_CLOCKS = 1023;  // barrier timestamps kept per step
 constexpr int CLOCK_T0 = MAX_CLOCKS + 1, CLOCK_WORDS = MAX_CLOCKS + 2;
 constexpr int STAT_WORDS = 16;    // collision ns, solve ns, then counters (pairs, contacts, manifolds, adjacency, incidences, dynamic, colours, rounds, launches, error)
 constexpr int C_STATS_NEXT = 13;  // counter word: next ring entry
+constexpr int C_CELLS = 15;       // counter word: slots of the sorted bodies handed out to cells (zero between steps)
 constexpr int C_HULL_PAIRS = 14;  // counter word: pairs deferred to the warp-per-pair hull narrowphase
 // Error bits
 constexpr uint32_t ERR_BARRIER_TIMEOUT = 1, ERR_ADJ_OVERFLOW = 2, ERR_INC_OVERFLOW = 4, ERR_DEPENDENCY_TIMEOUT = 8;
@@ -89,7 +90,7 @@ struct DWorld {
   // broadphase statics: large body indices, then (hi, lo, slot) no-collide triples sorted by (hi, lo)
   uint32_t *large, *nocollide;
   // broadphase scratch
-  uint32_t *keyA, *keyB, *valA, *valB, *radixHist;
+  uint32_t *keyA, *valA;
   int4* cell;
   uint32_t *cellStart, *cellEnd;
   float4* sortedPR;  // per sorted slot: position, bounding radius

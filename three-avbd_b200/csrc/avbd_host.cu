@@ -434,7 +434,6 @@ int avbd_world_create(const avbd_config* cfg, avbd_world** out) {
   DWorld& d = w->d;
   const uint32_t B = w->bodyCap;
   w->tableSize = pow2AtLeast(2ull * B);
-  w->sortTiles = (B + 8191) / 8192;
   w->maxSolveBlocks = solve_grid_blocks(w->device);
   w->sms = prop.multiProcessorCount;
   bool ok = true;
@@ -448,10 +447,7 @@ int avbd_world_create(const avbd_config* cfg, avbd_world** out) {
   }
   A(dalloc(w, &d.filters, B));
   A(dalloc(w, &d.keyA, B));
-  A(dalloc(w, &d.keyB, B));
   A(dalloc(w, &d.valA, B));
-  A(dalloc(w, &d.valB, B));
-  A(dalloc(w, &d.radixHist, size_t(w->tableSize) / 4096 + 2));
   A(dalloc(w, &d.cell, B));
   A(dalloc(w, &d.sortedPR, B));
   A(dalloc(w, &d.sortedCell, B));

@@ -40,7 +40,6 @@ struct avbd_world {
   std::string error;
   avbd_params params{};
   uint32_t bodyCap = 0, n = 0, jointCap = 0, nj = 0, pairCap = 0, tableSize = 0, hashSize = 0, incCap = 0, adjCap = 0;
-  uint32_t sortTiles = 0;
   DWorld d{};
   float4* staging = nullptr;  // body records for host transfers (10 float4 a body, capacity)
   int solveBlocks = 0, maxSolveBlocks = 0, sms = 0;  // the cooperative solve's grid (0: by the world's size; maxSolveBlocks: all co-resident)

@@ -1225,7 +1225,14 @@ __device__ void topologySolve(const DWorld& w, const StepParams& p, Team& team) 
   if (npairs > p.pairCap) npairs = p.pairCap;
   const uint32_t ncons = nj + npairs;
 
-  // A. degrees (adjStart[0, n] zeroed by the host)
+  // the warm-start table, past its last reader, emptied for the next step (a power of two words)
+  if constexpr (Team::kDataflow) {
+    uint4* h4 = reinterpret_cast<uint4*>(w.hash);
+    for (uint32_t i = tid; i < (p.hashMask + 1u) / 4u; i += T) h4[i] = make_uint4(0u, 0u, 0u, 0u);
+    if (p.hashMask < 3u && tid <= p.hashMask) w.hash[tid] = 0u;
+  }
+
+  // A. degrees (adjStart[0, n] is zero)
   for (uint32_t c = tid; c < ncons; c += T) {
     int ea, eb;
     uint32_t cnt;
@@ -1236,7 +1243,7 @@ __device__ void topologySolve(const DWorld& w, const StepParams& p, Team& team) 
   GSYNC
   if (!team_scan(w.adjStart, n + 1, w.scanScratch, team)) return;
   if (tid == 0) ctr[C_ADJ] = w.adjStart[n];
-  // B. fill (adjFill zeroed by the host), then each body's list sorted into its summation order and
+  // B. fill (adjFill is zero), then each body's list sorted into its summation order and
   // its row count (a joint is one row, a pair one per point)
   for (uint32_t c = tid; c < ncons; c += T) {
     int ea, eb;
@@ -1820,10 +1827,6 @@ cudaError_t launch_topology_solve(const DWorld& w, const StepParams& p, int bloc
   // the lane classes, and with them the order in which a body's rows are summed, do not follow the size
   pc.laneBudget = blocks <= 0 ? uint32_t(maxBlocks) * SOLVE_THREADS : 0u;
   if (blocks <= 0) blocks = one ? std::min<int>(sms, std::max<int>(1, int(p.n + 15u) / 16)) : maxBlocks;
-  cudaMemsetAsync(w.barrier, 0, 2 * sizeof(uint32_t), s);
-  cudaMemsetAsync(w.adjStart, 0, (size_t(p.n) + 1) * sizeof(uint32_t), s);
-  cudaMemsetAsync(w.adjFill, 0, (size_t(p.n) + 1) * sizeof(uint32_t), s);
-  cudaMemsetAsync(w.bucket, 0, BUCKET_WORDS * sizeof(uint32_t), s);
   DWorld wc = w;
   void* args[] = {&wc, &pc};
   const void* kernel = one ? (const void*)k_topology_solve<1> : (const void*)k_topology_solve<2>;
