@@ -58,3 +58,26 @@ def test_gpu_adjoint_matches_the_tape_adjoint(cuda_lib):
     # condition numbers near 1e7 and floored pivots: agreement to 1e-5 of the largest entry.
     assert worst_l < 1e-9 and worst_g < 1e-5
     adj.destroy()
+
+
+@pytest.mark.parametrize('bodies', [1, 15, 33, 70, 120])
+def test_every_block_size_gives_the_same_gradients(cuda_lib, bodies):
+    """One world, 200 and 300 of it (256, 128 and 64 threads a world; more bodies of one colour than are
+    solved together): the same sums in other orders, so the same gradients to the solves' conditioning
+    (1e7 times a double's rounding, of the largest entry), and the same in every copy."""
+    A = Oracle(tumbling_world(np.random.default_rng(bodies), bodies)).adjoint(4)
+    rec, p0 = A.export(), A.nominal()
+    target = np.tile([0.3, -0.2, 0.1, 0.0, 0.0, 0.0, 1.0], A.n)
+    grads = []
+    for worlds in (1, 200, 300):
+        adj = avbd_b200.Adjoint([rec] * worlds, checkpoint=3)
+        adj.set_target(np.tile(target, worlds))
+        loss, fin = adj.forward(np.tile(p0, worlds))
+        loss_b, g = adj.backward(np.tile(p0, worlds))
+        adj.destroy()
+        g = g.reshape(worlds, -1)
+        assert np.allclose(loss, loss[0], rtol=1e-12) and np.allclose(loss_b, loss, rtol=1e-12)
+        assert np.abs(g - g[0]).max() <= 1e-7 * np.abs(g[0]).max()
+        grads.append(g[0])
+    for g in grads[1:]:
+        assert np.abs(g - grads[0]).max() <= 1e-7 * np.abs(grads[0]).max()

@@ -24,9 +24,7 @@ using namespace avbd::adj;
 namespace {
 
 constexpr int ADJ_MAX_BODIES = 128;  // bodies of a world at most
-constexpr int ADJ_BLOCK = 64;        // threads a world (a block): bodies and points are strided over them
 constexpr int ADJ_MAX_POINTS = 1024;  // points of a world in one step at most
-constexpr int ADJ_BLOCKS_PER_SM = 8;  // worlds in flight per SM in the replay: registers capped at 128 a thread
 constexpr double PEN_MIN = 1.0, PEN_MAX = 1e10, PIVOT = 1e-5;
 
 // A body's primal solve at one iteration, kept by the segment recompute for the reverse sweep: its
@@ -84,6 +82,7 @@ struct AdjDev {
   QInv *irotI, *yrotI;  // the step-start and inertial rotations prepared for qsub
   double* pvz;
   D3 *lam, *pen, *lamP, *penP, *C0;  // world w's points at w * maxPts
+  double* fr;                        // the step's points' friction coefficients
   // checkpoints: every ck steps, the body state and the last step's points
   D3 *ckPos, *ckVel, *ckAng, *ckLam, *ckPen;
   D4* ckRot;
@@ -139,41 +138,42 @@ __device__ inline StepView viewOf(const AdjDev& D, int s, int w) {
 }
 
 constexpr int ADJ_MAX_COLORS = 64;
-constexpr int ADJ_GROUP = 16;  // bodies of one colour solved together, a thread each
+constexpr int ADJ_GROUP = 32;  // bodies of one colour solved together, a thread each
 constexpr int ADJ_ROW = 27;    // an incidence's share of its body's system: H's lower triangle, g
+constexpr int ADJ_OWN = 15;    // in the reverse sweep: its own body's pose, step-start pose and friction cotangents
 
 // The step's solve positions: its dynamic coloured bodies by colour, then by index; a colour's
 // bodies are positions s_colStart[c] .. s_colStart[c + 1], and their incidences (local point |
-// position << 16) are contiguous in s_inc, position p's at s_incStart[p] .. s_incStart[p + 1].
+// position << 16) are contiguous in incList(), position p's at s_incStart[p] .. s_incStart[p + 1].
 __shared__ int s_colStart[ADJ_MAX_COLORS + 1];
 __shared__ int s_colBody[ADJ_MAX_BODIES];
 __shared__ int s_posOf[ADJ_MAX_BODIES];
 __shared__ int s_nSolved;
 __shared__ int s_incStart[ADJ_MAX_BODIES + 1];
-__shared__ int s_inc[2 * ADJ_MAX_POINTS];
 __shared__ int s_color[ADJ_MAX_BODIES];
-// Dynamic shared memory: a chunk of incidences, a row each (its share of the body's system, or its
-// own-body cotangents), then, in the reverse sweep, a group's bodies: step, cotangent of g, and for a
-// floored factorization the cotangents of H and L
+// Dynamic shared memory: a chunk of incidences, a row each (a block's threads; its share of the body's
+// system, or its own-body cotangents), a group's sums of the rows, in the reverse sweep the group's
+// bodies (step, cotangent of g), then the step's points (bodies a | b << 8, manifold) and incidences.
 struct BodyVjp {
   double delta[6], w[6];
   int floored;
 };
 extern __shared__ __align__(16) double s_dyn[];
-constexpr size_t ADJ_SMEM_ROWS = sizeof(double) * ADJ_BLOCK * ADJ_ROW;
-constexpr size_t ADJ_SMEM_FORWARD = ADJ_SMEM_ROWS, ADJ_SMEM_BACKWARD = ADJ_SMEM_ROWS + sizeof(BodyVjp) * ADJ_GROUP;
 __device__ inline double* rowOf(int i) { return s_dyn + size_t(i) * ADJ_ROW; }
-// In the reverse sweep an incidence's row is its own body's cotangents (14); a group slot's sums of
-// them follow the rows, so that they stay in shared memory rather than registers across the
-// incidences' long evaluation
-constexpr int ADJ_OWN = 14;
 __device__ inline double* ownRow(int i) { return s_dyn + size_t(i) * ADJ_OWN; }
-__device__ inline double* ownSum(int slot) { return s_dyn + size_t(ADJ_BLOCK) * ADJ_OWN + size_t(slot) * ADJ_OWN; }
-static_assert(size_t(ADJ_BLOCK + ADJ_GROUP) * ADJ_OWN <= size_t(ADJ_BLOCK) * ADJ_ROW, "the reverse rows and sums fit in the rows");
-__device__ inline BodyVjp* bodyVjp() { return reinterpret_cast<BodyVjp*>(s_dyn + size_t(ADJ_BLOCK) * ADJ_ROW); }
-// While the incidence is built the rows are free: the step's points' bodies (world-local) go there
-__device__ inline int2* pointBodies() { return reinterpret_cast<int2*>(s_dyn); }
-static_assert(sizeof(int2) * ADJ_MAX_POINTS <= ADJ_SMEM_ROWS, "a step's point bodies fit in the rows");
+__device__ inline double* groupSums() { return s_dyn + size_t(blockDim.x) * ADJ_ROW; }
+__device__ inline BodyVjp* bodyVjp() { return reinterpret_cast<BodyVjp*>(groupSums() + ADJ_GROUP * ADJ_ROW); }
+__device__ inline int* pointBodies() { return reinterpret_cast<int*>(bodyVjp() + ADJ_GROUP); }
+__device__ inline int* pointManifold(int maxPts) { return pointBodies() + maxPts; }
+__device__ inline int* incList(int maxPts) { return pointBodies() + 2 * maxPts; }
+constexpr size_t adjSharedBytes(int threads, int maxPts) {
+  return sizeof(double) * (size_t(threads) + ADJ_GROUP) * ADJ_ROW + sizeof(BodyVjp) * ADJ_GROUP + sizeof(int) * 4 * size_t(maxPts);
+}
+static_assert(adjSharedBytes(256, ADJ_MAX_POINTS) <= 99 * 1024, "a block's shared memory");
+__device__ inline int2 bodiesOf(int lk) {
+  const int ab = pointBodies()[lk];
+  return make_int2(ab & 0xff, ab >> 8);
+}
 // Group slot i's floored-factorization cotangents (H's, then L's): global, as floored pivots are rare
 __device__ inline double* floorHb(const AdjDev& D, int i) { return D.floorWork + (size_t(blockIdx.x) * ADJ_GROUP + i) * 72; }
 
@@ -208,11 +208,16 @@ __device__ void buildIncidence(const AdjDev& D, const StepView& v) {
   for (int i = tid; i <= s_nSolved; i += blockDim.x) s_incStart[i] = 0;
   // the step's points' bodies, once, for the counts and the per-body fill
   const int np = v.p1 - v.p0;
-  int2* s_ptAB = pointBodies();
-  for (int lk = tid; lk < np; lk += blockDim.x) s_ptAB[lk] = D.manAB[D.ptMan[v.p0 + lk]];
+  int* s_inc = incList(D.maxPts);
+  for (int lk = tid; lk < np; lk += blockDim.x) {
+    const int m = D.ptMan[v.p0 + lk];
+    const int2 ab = D.manAB[m];
+    pointBodies()[lk] = ab.x | (ab.y << 8);
+    pointManifold(D.maxPts)[lk] = m;
+  }
   __syncthreads();
   for (int lk = tid; lk < np; lk += blockDim.x) {
-    const int2 ab = s_ptAB[lk];
+    const int2 ab = bodiesOf(lk);
     const int pa = s_posOf[ab.x], pb = s_posOf[ab.y];
     if (pa >= 0) atomicAdd(&s_incStart[pa + 1], 1);
     if (pb >= 0) atomicAdd(&s_incStart[pb + 1], 1);
@@ -226,7 +231,7 @@ __device__ void buildIncidence(const AdjDev& D, const StepView& v) {
     const int lb = s_colBody[p];
     int o = s_incStart[p];
     for (int lk = 0; lk < np; lk++) {
-      const int2 ab = s_ptAB[lk];
+      const int2 ab = bodiesOf(lk);
       if (ab.x == lb || ab.y == lb) s_inc[o++] = lk | (p << 16);
     }
   }
@@ -243,9 +248,8 @@ struct PointEval {
   double fs, bd, fr;
   bool clamped;
 };
-__device__ inline void evalPoint(const AdjDev& D, int k, D3 xa, D4 qa, D3 xa0, const QInv& qa0, D3 xb, D4 qb, D3 xb0, const QInv& qb0, D3 c0, D3 lam, D3 pen, double fr,
+__device__ inline void evalPoint(const AdjDev& D, int k, const D3* B, D3 xa, D4 qa, D3 xa0, const QInv& qa0, D3 xb, D4 qb, D3 xb0, const QInv& qb0, D3 c0, D3 lam, D3 pen, double fr,
                                  PointEval& e) {
-  const D3* B = D.basis + 3 * D.ptMan[k];
   e.rAW = rotate(qa, D.anchor[2 * k]);
   e.rBW = rotate(qb, D.anchor[2 * k + 1]);
   e.dAL = xa - xa0;
@@ -297,9 +301,8 @@ __device__ inline void evalFVjp(const PointEval& e, D3 lam, D3 pen, D3 gF, D3& g
 }
 
 // The cotangents of the poses, step-start poses and C0 from the cotangent of C
-__device__ inline void evalCVjp(const AdjDev& D, int k, D4 qa, D4 qa0, const QInv& ia0, D4 qb, D4 qb0, const QInv& ib0, const PointEval& e, D3 gC, D3& gXa, D4& gQa, D3& gXa0, D4& gQa0,
+__device__ inline void evalCVjp(const AdjDev& D, int k, const D3* B, D4 qa, D4 qa0, const QInv& ia0, D4 qb, D4 qb0, const QInv& ib0, const PointEval& e, D3 gC, D3& gXa, D4& gQa, D3& gXa0, D4& gQa0,
                                 D3& gXb, D4& gQb, D3& gXb0, D4& gQb0, D3& gC0) {
-  const D3* B = D.basis + 3 * D.ptMan[k];
   D3 gdAL{0, 0, 0}, gdAA{0, 0, 0}, gdBL{0, 0, 0}, gdBA{0, 0, 0}, grA{0, 0, 0}, grB{0, 0, 0};
   for (int c = 0; c < 3; c++) {
     double g = comp(gC, c);
@@ -329,18 +332,17 @@ __device__ inline void incidenceRows(const AdjDev& D, const StepView& v, int wpt
                                      double* row) {
   const int lk = entry & 0xffff, k = v.p0 + lk;
   const int gb = v.b0 + s_colBody[entry >> 16];
-  const int2 ab = D.manAB[D.ptMan[k]];
+  const int2 ab = bodiesOf(lk);
+  const D3* B = D.basis + 3 * size_t(pointManifold(D.maxPts)[lk]);
   const int a = v.b0 + ab.x, b = v.b0 + ab.y;
   D3 xa, xb;
   D4 qa, qb;
   poseOf(a, xa, qa);
   poseOf(b, xb, qb);
   PointEval e;
-  evalPoint(D, k, xa, qa, D.ipos[a], D.irotI[a], xb, qb, D.ipos[b], D.irotI[b], D.C0[wpt + lk], lamCur[wpt + lk], penCur[wpt + lk],
-            sqrt(mu(D, a) * mu(D, b)), e);
+  evalPoint(D, k, B, xa, qa, D.ipos[a], D.irotI[a], xb, qb, D.ipos[b], D.irotI[b], D.C0[wpt + lk], lamCur[wpt + lk], penCur[wpt + lk], D.fr[wpt + lk], e);
   const double sg = gb == a ? 1.0 : -1.0;
   const D3 rr = gb == a ? e.rAW : e.rBW;
-  const D3* B = D.basis + 3 * D.ptMan[k];
   double h[21], r[6];
   for (int i = 0; i < 21; i++) h[i] = 0.0;
   for (int i = 0; i < 6; i++) r[i] = 0.0;
@@ -358,23 +360,36 @@ __device__ inline void incidenceRows(const AdjDev& D, const StepView& v, int wpt
   for (int i = 0; i < 6; i++) row[21 + i] = r[i];
 }
 
-// The bodies at positions g0..g1 (thread tid: position g0 + tid) sum their incidences' rows, a chunk
-// of incidences at a time (one per thread), in incidence order
+// The replay and the reverse sweep are bound by the latency of their double-precision chains. What kept
+// them longer than need be: sixteen threads adding up a group's rows, 27 values one after another; groups
+// of 16 bodies, so that a colour's solves ran in two or more rounds; a square root a point and visit for a
+// friction coefficient that is fixed for the step; dependent loads for a point's bodies and manifold;
+// global atomics for values that no other thread touches. 16 worlds: 9.95 ms, now 4.44; 1024: 38.3, now
+// 29.0 (forward and backward, the sizes at blockThreads).
+//
+// The sums over the incidences of the bodies at positions g0..g1 of `width` values each, row u of the
+// chunk starting at ch being row(u - ch): a thread a (body, value), in incidence order
+template <class RowOf>
+__device__ inline void addChunk(int g0, int g1, int ch, bool first, int width, RowOf row) {
+  double* sums = groupSums();
+  for (int t = threadIdx.x; t < (g1 - g0) * width; t += blockDim.x) {
+    const int p = g0 + t / width, i = t % width;
+    double acc = first ? 0.0 : sums[t];
+    const int u0 = max(s_incStart[p], ch), u1 = min(s_incStart[p + 1], ch + int(blockDim.x));
+    for (int u = u0; u < u1; u++) acc += row(u - ch)[i];
+    sums[t] = acc;
+  }
+}
+// The bodies at positions g0..g1 sum their incidences' rows, a chunk of incidences at a time (one per
+// thread): position p's sums at groupSums() + (p - g0) ADJ_ROW
 template <class PoseOf>
-__device__ inline void groupRows(const AdjDev& D, const StepView& v, int wpt, int g0, int g1, const D3* lamCur, const D3* penCur, PoseOf poseOf,
-                                 double* acc) {
+__device__ inline void groupRows(const AdjDev& D, const StepView& v, int wpt, int g0, int g1, const D3* lamCur, const D3* penCur, PoseOf poseOf) {
   const int tid = threadIdx.x;
-  for (int i = 0; i < ADJ_ROW; i++) acc[i] = 0.0;
   const int i0 = s_incStart[g0], i1 = s_incStart[g1];
-  for (int ch = i0; ch < i1; ch += blockDim.x) {
-    if (ch + tid < i1) incidenceRows(D, v, wpt, s_inc[ch + tid], lamCur, penCur, poseOf, rowOf(tid));
+  for (int ch = i0; ch < i1 || ch == i0; ch += blockDim.x) {
+    if (ch + tid < i1) incidenceRows(D, v, wpt, incList(D.maxPts)[ch + tid], lamCur, penCur, poseOf, rowOf(tid));
     __syncthreads();
-    if (tid < g1 - g0) {
-      const int p = g0 + tid;
-      const int u0 = max(s_incStart[p], ch), u1 = min(s_incStart[p + 1], ch + int(blockDim.x));
-      for (int u = u0; u < u1; u++)
-        for (int i = 0; i < ADJ_ROW; i++) acc[i] += rowOf(u - ch)[i];
-    }
+    addChunk(g0, g1, ch, ch == i0, ADJ_ROW, [](int i) { return rowOf(i); });
     __syncthreads();
   }
 }
@@ -428,10 +443,11 @@ __device__ void stepForward(const AdjDev& D, int s, int w, int slot) {
     }
     D3 lw = l * (D.alpha * D.gamma), pw;
     for (int c = 0; c < 3; c++) setComp(pw, c, fmin(fmax(comp(pe, c) * D.gamma, PEN_MIN), PEN_MAX));
-    int2 ab = D.manAB[D.ptMan[k]];
+    int2 ab = bodiesOf(lk);
     int a = v.b0 + ab.x, b = v.b0 + ab.y;
+    D.fr[wpt + lk] = sqrt(mu(D, a) * mu(D, b));
     D3 d = (rotate(D.rot[a], D.anchor[2 * k]) + D.pos[a]) - (rotate(D.rot[b], D.anchor[2 * k + 1]) + D.pos[b]);
-    const D3* B = D.basis + 3 * D.ptMan[k];
+    const D3* B = D.basis + 3 * size_t(pointManifold(D.maxPts)[lk]);
     D3 c0{dot(B[0], d) + D.margin, dot(B[1], d), dot(B[2], d)};
     D.lam[wpt + lk] = lw;
     D.pen[wpt + lk] = pw;
@@ -485,13 +501,12 @@ __device__ void stepForward(const AdjDev& D, int s, int w, int slot) {
     for (int c = 0; c < v.ncol; c++) {  // the colour's bodies in groups, a thread each
       for (int g0 = s_colStart[c]; g0 < s_colStart[c + 1]; g0 += ADJ_GROUP) {
         const int g1 = min(g0 + ADJ_GROUP, s_colStart[c + 1]);
-        double acc[ADJ_ROW];
-        groupRows(D, v, wpt, g0, g1, D.lam, D.pen, livePose, acc);
+        groupRows(D, v, wpt, g0, g1, D.lam, D.pen, livePose);
         if (threadIdx.x < g1 - g0) {
           const int gb = v.b0 + s_colBody[g0 + threadIdx.x];
           Sys6 S;
           double rhs[6], dx[6];
-          bodySystem(D, gb, acc, livePose, S, rhs);
+          bodySystem(D, gb, groupSums() + size_t(threadIdx.x) * ADJ_ROW, livePose, S, rhs);
           LDLT6 F;
           const int floored = factor6(S, F, PIVOT);
           solve6(F, rhs, dx);
@@ -517,11 +532,11 @@ __device__ void stepForward(const AdjDev& D, int s, int w, int slot) {
     // duals (manifold.ts:202-217)
     for (int lk = threadIdx.x; lk < np; lk += blockDim.x) {
       int k = v.p0 + lk;
-      int2 ab = D.manAB[D.ptMan[k]];
+      int2 ab = bodiesOf(lk);
       int a = v.b0 + ab.x, b = v.b0 + ab.y;
       PointEval e;
-      evalPoint(D, k, D.pos[a], D.rot[a], D.ipos[a], D.irotI[a], D.pos[b], D.rot[b], D.ipos[b], D.irotI[b], D.C0[wpt + lk], D.lam[wpt + lk], D.pen[wpt + lk],
-                sqrt(mu(D, a) * mu(D, b)), e);
+      evalPoint(D, k, D.basis + 3 * size_t(pointManifold(D.maxPts)[lk]), D.pos[a], D.rot[a], D.ipos[a], D.irotI[a], D.pos[b], D.rot[b], D.ipos[b], D.irotI[b],
+                D.C0[wpt + lk], D.lam[wpt + lk], D.pen[wpt + lk], D.fr[wpt + lk], e);
       D3 pen = D.pen[wpt + lk];
       if (e.F.x < 0.0) pen.x = fmin(pen.x + D.beta * fabs(e.C.x), PEN_MAX);
       if (e.fs <= e.bd) {
@@ -621,7 +636,7 @@ __device__ inline int pointsBefore(const AdjDev& D, int s, int w) {  // the last
 
 __device__ void worldLoss(const AdjDev& D, int w) {
   const int b0 = D.bodyFirst[w], nb = D.bodyFirst[w + 1] - b0;
-  __shared__ double s_loss[ADJ_BLOCK];
+  double* s_loss = s_dyn;  // the rows are free here
   double l = 0.0;
   for (int bi = threadIdx.x; bi < nb; bi += blockDim.x) {
     int gb = b0 + bi;
@@ -637,6 +652,7 @@ __device__ void worldLoss(const AdjDev& D, int w) {
       o[0] = x.x; o[1] = x.y; o[2] = x.z; o[3] = q.x; o[4] = q.y; o[5] = q.z; o[6] = q.w;
     }
   }
+  __syncthreads();
   s_loss[threadIdx.x] = l;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -647,7 +663,9 @@ __device__ void worldLoss(const AdjDev& D, int w) {
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(ADJ_BLOCK, ADJ_BLOCKS_PER_SM) k_adj_forward(AdjDev D) {
+// Both kernels come in blocks of 64, 128 or 256 threads a world (blockThreads, below)
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, 512 / kThreads) k_adj_forward(AdjDev D) {
   const int w = blockIdx.x;
   loadInitial(D, w);
   for (int s = 0; s < D.K; s++) {
@@ -671,20 +689,20 @@ __device__ inline void incidenceVjp(const AdjDev& D, const StepView& v, int wpt,
   const D3 dL{bv.delta[0], bv.delta[1], bv.delta[2]}, dA{bv.delta[3], bv.delta[4], bv.delta[5]};
   const D3 wl{bv.w[0], bv.w[1], bv.w[2]}, wa{bv.w[3], bv.w[4], bv.w[5]};
   const int floored = bv.floored;
-  const int2 ab = D.manAB[D.ptMan[k]];
+  const int2 ab = bodiesOf(lk);
+  const D3* B = D.basis + 3 * size_t(pointManifold(D.maxPts)[lk]);
   const int a = v.b0 + ab.x, b = v.b0 + ab.y;
   D3 xa, xb;
   D4 qa, qb;
   poseOf(a, xa, qa);
   poseOf(b, xb, qb);
-  const double fr = sqrt(mu(D, a) * mu(D, b));
+  const double fr = D.fr[wpt + lk];
   PointEval e;
   const D3 lamv = lamIn[wpt + lk], penv = penIn[wpt + lk];
-  evalPoint(D, k, xa, qa, D.ipos[a], D.irotI[a], xb, qb, D.ipos[b], D.irotI[b], D.C0[wpt + lk], lamv, penv, fr, e);
+  evalPoint(D, k, B, xa, qa, D.ipos[a], D.irotI[a], xb, qb, D.ipos[b], D.irotI[b], D.C0[wpt + lk], lamv, penv, fr, e);
   const bool isA = gb == a;
   const double sg = isA ? 1.0 : -1.0;
   const D3 r = isA ? e.rAW : e.rBW;
-  const D3* B = D.basis + 3 * D.ptMan[k];
   D3 gF{0, 0, 0}, gPen{0, 0, 0}, gr{0, 0, 0};
   for (int cc = 0; cc < 3; cc++) {
     const D3 l = B[cc] * sg;
@@ -719,7 +737,7 @@ __device__ inline void incidenceVjp(const AdjDev& D, const StepView& v, int wpt,
   evalFVjp(e, lamv, penv, gF, gC, gLam, gPen, gFr);
   D3 gXa{0, 0, 0}, gXb{0, 0, 0}, gXa0{0, 0, 0}, gXb0{0, 0, 0}, gC0{0, 0, 0};
   D4 gQa{0, 0, 0, 0}, gQb{0, 0, 0, 0}, gQa0{0, 0, 0, 0}, gQb0{0, 0, 0, 0};
-  evalCVjp(D, k, qa, D.irot[a], D.irotI[a], qb, D.irot[b], D.irotI[b], e, gC, gXa, gQa, gXa0, gQa0, gXb, gQb, gXb0, gQb0, gC0);
+  evalCVjp(D, k, B, qa, D.irot[a], D.irotI[a], qb, D.irot[b], D.irotI[b], e, gC, gXa, gQa, gXa0, gQa0, gXb, gQb, gXb0, gQb0, gC0);
   // the lever arm r = R(q_own) r_local
   if (isA) gQa += rotateVjpQ(qa, D.anchor[2 * k], gr);
   else gQb += rotateVjpQ(qb, D.anchor[2 * k + 1], gr);
@@ -732,13 +750,15 @@ __device__ inline void incidenceVjp(const AdjDev& D, const StepView& v, int wpt,
     atomicAdd3(&D.gIpos[other], isA ? gXb0 : gXa0);
     atomicAdd4(&D.gIrot[other], isA ? gQb0 : gQa0);
   }
-  atomicAdd3(&D.gLam[wpt + lk], gLam);
-  atomicAdd3(&D.gPen[wpt + lk], gPen);
-  atomicAdd3(&D.gC0[wpt + lk], gC0);
+  // a point has one incidence in a colour: nothing else touches its values here
+  D.gLam[wpt + lk] += gLam;
+  D.gPen[wpt + lk] += gPen;
+  D.gC0[wpt + lk] += gC0;
+  out[14] = 0.0;
   if (gFr != 0.0 && fr > 0.0) {
-    double ma = mu(D, a), mb = mu(D, b);
-    if (D.dynamic[a]) atomicAdd(&D.gMu[a], gFr * mb / (2.0 * fr));
-    if (D.dynamic[b]) atomicAdd(&D.gMu[b], gFr * ma / (2.0 * fr));
+    const double half = gFr / (2.0 * fr);
+    out[14] = half * mu(D, other);
+    if (D.dynamic[other]) atomicAdd(&D.gMu[other], half * mu(D, gb));
   }
   out[0] = oX.x, out[1] = oX.y, out[2] = oX.z;
   out[3] = oQ.x, out[4] = oQ.y, out[5] = oQ.z, out[6] = oQ.w;
@@ -801,24 +821,16 @@ __device__ void primalGroupVjp(const AdjDev& D, const StepView& v, int wpt, int 
     bv.floored = floored;
   }
   __syncthreads();
-  // the incidences' cotangents; each body sums its own
-  if (tid < nbg)
-    for (int i = 0; i < ADJ_OWN; i++) ownSum(tid)[i] = 0.0;
+  // the incidences' cotangents; each body's own are summed
   const int i0 = s_incStart[g0], i1 = s_incStart[g1];
-  for (int ch = i0; ch < i1; ch += blockDim.x) {
-    if (ch + tid < i1) incidenceVjp(D, v, wpt, s_inc[ch + tid], g0, lamIn, penIn, poseOf, ownRow(tid));
+  for (int ch = i0; ch < i1 || ch == i0; ch += blockDim.x) {
+    if (ch + tid < i1) incidenceVjp(D, v, wpt, incList(D.maxPts)[ch + tid], g0, lamIn, penIn, poseOf, ownRow(tid));
     __syncthreads();
-    if (tid < nbg) {
-      const int p = g0 + tid;
-      const int u0 = max(s_incStart[p], ch), u1 = min(s_incStart[p + 1], ch + int(blockDim.x));
-      double* own = ownSum(tid);
-      for (int u = u0; u < u1; u++)
-        for (int i = 0; i < ADJ_OWN; i++) own[i] += ownRow(u - ch)[i];
-    }
+    addChunk(g0, g1, ch, ch == i0, ADJ_OWN, [](int i) { return ownRow(i); });
     __syncthreads();
   }
   if (tid < nbg) {
-    const double* own = ownSum(tid);
+    const double* own = groupSums() + size_t(tid) * ADJ_OWN;
     const int gb = v.b0 + s_colBody[g0 + tid];
     const BodyVjp& bv = bodyVjp()[tid];
     D3 x;
@@ -858,6 +870,7 @@ __device__ void primalGroupVjp(const AdjDev& D, const StepView& v, int wpt, int 
     D.gIpos[gb] += D3{own[7], own[8], own[9]};
     D.gIrot[gb] += D4{own[10], own[11], own[12], own[13]};
     D.gMass[gb] += gM;
+    D.gMu[gb] += own[14];
   }
   __syncthreads();
 }
@@ -868,14 +881,15 @@ __device__ void dualVjp(const AdjDev& D, const StepView& v, int wpt, int it, int
   const size_t sn = (size_t)(it + 1) * D.nb;
   const D3* lamIn = D.snLam + (size_t)it * D.W * D.maxPts;
   const D3* penIn = D.snPen + (size_t)it * D.W * D.maxPts;
-  int2 ab = D.manAB[D.ptMan[k]];
+  int2 ab = bodiesOf(lk);
+  const D3* B = D.basis + 3 * size_t(pointManifold(D.maxPts)[lk]);
   int a = v.b0 + ab.x, b = v.b0 + ab.y;
   D3 xa = D.snPos[sn + a], xb = D.snPos[sn + b];
   D4 qa = D.snRot[sn + a], qb = D.snRot[sn + b];
-  double fr = sqrt(mu(D, a) * mu(D, b));
+  double fr = D.fr[wpt + lk];
   D3 lamv = lamIn[wpt + lk], penv = penIn[wpt + lk];
   PointEval e;
-  evalPoint(D, k, xa, qa, D.ipos[a], D.irotI[a], xb, qb, D.ipos[b], D.irotI[b], D.C0[wpt + lk], lamv, penv, fr, e);
+  evalPoint(D, k, B, xa, qa, D.ipos[a], D.irotI[a], xb, qb, D.ipos[b], D.irotI[b], D.C0[wpt + lk], lamv, penv, fr, e);
   D3 gLamOut = D.gLam[wpt + lk], gPenOut = D.gPen[wpt + lk];
   D3 gPen{0, 0, 0}, gC{0, 0, 0}, gLam{0, 0, 0};
   // pen' = min(pen + beta |C|, MAX) where the ramp applies, else pen
@@ -898,7 +912,7 @@ __device__ void dualVjp(const AdjDev& D, const StepView& v, int wpt, int it, int
   evalFVjp(e, lamv, penv, gLamOut, gC, gLam, gPen, gFr);
   D3 gXa{0, 0, 0}, gXb{0, 0, 0}, gXa0{0, 0, 0}, gXb0{0, 0, 0}, gC0{0, 0, 0};
   D4 gQa{0, 0, 0, 0}, gQb{0, 0, 0, 0}, gQa0{0, 0, 0, 0}, gQb0{0, 0, 0, 0};
-  evalCVjp(D, k, qa, D.irot[a], D.irotI[a], qb, D.irot[b], D.irotI[b], e, gC, gXa, gQa, gXa0, gQa0, gXb, gQb, gXb0, gQb0, gC0);
+  evalCVjp(D, k, B, qa, D.irot[a], D.irotI[a], qb, D.irot[b], D.irotI[b], e, gC, gXa, gQa, gXa0, gQa0, gXb, gQb, gXb0, gQb0, gC0);
   if (D.dynamic[a]) {
     atomicAdd3(&D.gPos[a], gXa);
     atomicAdd4(&D.gRot[a], gQa);
@@ -973,7 +987,11 @@ __device__ void stepBackward(const AdjDev& D0, int s, int w, size_t slot) {
     D.gAng[gb] = D3{0, 0, 0};
     D.gPvz[gb] = 0.0;
   }
-  for (int lk = threadIdx.x; lk < np; lk += blockDim.x) D.gC0[wpt + lk] = D3{0, 0, 0};
+  for (int lk = threadIdx.x; lk < np; lk += blockDim.x) {
+    D.gC0[wpt + lk] = D3{0, 0, 0};
+    const int2 ab = bodiesOf(lk);
+    D.fr[wpt + lk] = sqrt(mu(D, v.b0 + ab.x) * mu(D, v.b0 + ab.y));
+  }
   __syncthreads();
   for (int it = D.I - 1; it >= 0; it--) {
     for (int lk = threadIdx.x; lk < np; lk += blockDim.x) dualVjp(D, v, wpt, it, v.p0 + lk);
@@ -998,9 +1016,9 @@ __device__ void stepBackward(const AdjDev& D0, int s, int w, size_t slot) {
       atomicAdd3(&D.gLamP[wpt + plk], gl * (D.alpha * D.gamma));  // two points may warm-start from one
       atomicAdd3(&D.gPenP[wpt + plk], gpp);
     }
-    int2 ab = D.manAB[D.ptMan[k]];
+    int2 ab = bodiesOf(lk);
     int a = v.b0 + ab.x, b = v.b0 + ab.y;
-    const D3* B = D.basis + 3 * D.ptMan[k];
+    const D3* B = D.basis + 3 * size_t(pointManifold(D.maxPts)[lk]);
     D3 gc0 = D.gC0[wpt + lk];
     D3 gd = B[0] * gc0.x + B[1] * gc0.y + B[2] * gc0.z;
     if (D.dynamic[a]) {
@@ -1050,9 +1068,10 @@ __device__ void stepBackward(const AdjDev& D0, int s, int w, size_t slot) {
   __syncthreads();
 }
 
-// The reverse sweep's incidence cotangents hold more live state than 128 registers: 4 worlds an SM
-// at up to 255 registers beat 8 at 128 with spills
-__global__ void __launch_bounds__(ADJ_BLOCK, 4) k_adj_backward(const AdjDev D) {
+// The reverse sweep's incidence cotangents hold more live state than 128 registers: 256 threads an SM
+// at up to 255 registers beat 512 at 128 with spills
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, 256 / kThreads) k_adj_backward(const AdjDev D) {
   const int w = blockIdx.x;
   const int b0 = D.bodyFirst[w], nb = D.bodyFirst[w + 1] - b0;
   const int wpt = w * D.maxPts;
@@ -1105,6 +1124,14 @@ __global__ void __launch_bounds__(ADJ_BLOCK, 4) k_adj_backward(const AdjDev D) {
 
 }  // namespace
 
+// Threads a world. A world is a serial chain of colours, its links a round of incidences (or points)
+// over its threads and a solve a body: alone on its SM it is faster the fewer rounds it takes; where
+// worlds fill the SMs (registers cap both kernels' threads an SM, not their blocks) small blocks let
+// one world's solves run under another's rounds. Forward and backward, 10 iterations, at 64, 128 and
+// 256 threads: 16 worlds of 24 boxes over 12 steps 6.95, 4.59 and 4.45 ms; 1024 of 64 boxes over 8 steps
+// 29.6, 32.7 and 34.4 ms.
+static int blockThreads(int worlds) { return worlds <= 148 ? 256 : worlds <= 296 ? 128 : 64; }
+
 struct avbd_adjoint {
   int device = 0;
   std::string error;
@@ -1115,6 +1142,17 @@ struct avbd_adjoint {
   uint64_t manifolds = 0, points = 0;
   bool forwardDone = false;  // the checkpoints hold the forward of lastParams
   std::vector<double> lastParams;
+  int threads = 64;  // threads a world
+  const void* forwardKernel() const {
+    return threads == 64 ? (const void*)k_adj_forward<64> : threads == 128 ? (const void*)k_adj_forward<128> : (const void*)k_adj_forward<256>;
+  }
+  const void* backwardKernel() const {
+    return threads == 64 ? (const void*)k_adj_backward<64> : threads == 128 ? (const void*)k_adj_backward<128> : (const void*)k_adj_backward<256>;
+  }
+  cudaError_t launch(const void* kernel) {
+    void* args[] = {&d};
+    return cudaLaunchKernel(kernel, dim3(W), dim3(threads), args, adjSharedBytes(threads, d.maxPts), nullptr);
+  }
 };
 
 namespace {
@@ -1144,12 +1182,10 @@ bool aupload(avbd_adjoint* a, const T** dst, const T* src, size_t n) {
 // The replay's working buffers, checkpoints, snapshots and cotangents (D's sizes set)
 bool adjAllocWork(avbd_adjoint* a) {
   AdjDev& D = a->d;
-  // shared memory sized for the blocks of several worlds on one SM
-  if (cudaFuncSetAttribute(k_adj_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ADJ_SMEM_FORWARD)) != cudaSuccess ||
-      cudaFuncSetAttribute(k_adj_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ADJ_SMEM_BACKWARD)) != cudaSuccess ||
-      cudaFuncSetAttribute(k_adj_forward, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess ||
-      cudaFuncSetAttribute(k_adj_backward, cudaFuncAttributePreferredSharedMemoryCarveout, 100) != cudaSuccess)
-    return false;
+  a->threads = blockThreads(D.W);
+  const int bytes = int(adjSharedBytes(a->threads, D.maxPts));
+  for (const void* k : {a->forwardKernel(), a->backwardKernel()})
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
   const size_t W = size_t(D.W), K = size_t(D.K), nb = size_t(D.nb);
   bool ok = true;
   const size_t WP = W * size_t(D.maxPts), segs = (K + D.ck - 1) / D.ck, I1 = size_t(D.I) + 1;
@@ -1162,6 +1198,7 @@ bool adjAllocWork(avbd_adjoint* a) {
   for (D4** p : {&D.rot, &D.irot, &D.yrot, &D.gRot, &D.gIrot, &D.gYrot}) ok = ok && aalloc(a, p, nb);
   ok = ok && aalloc(a, &D.irotI, nb) && aalloc(a, &D.yrotI, nb);
   for (double** p : {&D.pvz, &D.gPvz, &D.gMass, &D.gMu}) ok = ok && aalloc(a, p, nb);
+  ok = ok && aalloc(a, &D.fr, WP);
   for (D3** p : {&D.lam, &D.pen, &D.lamP, &D.penP, &D.C0, &D.gLam, &D.gPen, &D.gLamP, &D.gPenP, &D.gC0}) ok = ok && aalloc(a, p, WP);
   ok = ok && aalloc(a, &D.ckPos, segs * nb) && aalloc(a, &D.ckVel, segs * nb) && aalloc(a, &D.ckAng, segs * nb) && aalloc(a, &D.ckRot, segs * nb) &&
        aalloc(a, &D.ckPvz, segs * nb) && aalloc(a, &D.ckLam, segs * WP) && aalloc(a, &D.ckPen, segs * WP);
@@ -1473,8 +1510,7 @@ int avbd_adjoint_forward(avbd_adjoint* a, const double* params, double* loss, do
   cudaSetDevice(a->device);
   int r = adjParams(a, params);
   if (r) return r;
-  k_adj_forward<<<a->W, ADJ_BLOCK, ADJ_SMEM_FORWARD>>>(a->d);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = a->launch(a->forwardKernel());
   if (e != cudaSuccess) return afail(a, AVBD_ERR_CUDA, std::string("replay launch: ") + cudaGetErrorString(e));
   e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return afail(a, AVBD_ERR_CUDA, cudaGetErrorString(e));
@@ -1492,13 +1528,11 @@ int avbd_adjoint_backward(avbd_adjoint* a, const double* params, double* grad, d
   int r = adjParams(a, params);
   if (r) return r;
   if (!a->forwardDone) {  // the checkpoints come from a forward with these params
-    k_adj_forward<<<a->W, ADJ_BLOCK, ADJ_SMEM_FORWARD>>>(a->d);
-    cudaError_t e0 = cudaGetLastError();
+    cudaError_t e0 = a->launch(a->forwardKernel());
     if (e0 != cudaSuccess) return afail(a, AVBD_ERR_CUDA, std::string("replay launch: ") + cudaGetErrorString(e0));
   }
   a->forwardDone = false;
-  k_adj_backward<<<a->W, ADJ_BLOCK, ADJ_SMEM_BACKWARD>>>(a->d);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = a->launch(a->backwardKernel());
   if (e != cudaSuccess) return afail(a, AVBD_ERR_CUDA, std::string("reverse launch: ") + cudaGetErrorString(e));
   e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return afail(a, AVBD_ERR_CUDA, cudaGetErrorString(e));
