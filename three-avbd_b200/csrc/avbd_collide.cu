@@ -1686,9 +1686,17 @@ __global__ void __launch_bounds__(128) k_narrowphase(DWorld w, StepParams p) {
 
 // --- batched worlds: one block per world ------------------------------------------------------------------
 // A world of a batch holds at most a few hundred bodies: its pairs are found by testing every pair
-// of bodies against the broadphase rule (the same set the grid walk finds), then collided.
+// of bodies against the broadphase rule (the same set the grid walk finds), then collided. Up to
+// BATCH_STAGE bodies the test runs on spheres in shared memory and the pairs that pass it get the full
+// test on full warps: a thread a pair read seven scattered words for every test and ran the full one on
+// the one or two lanes of a warp that came to it (96 worlds a step 597 us, now 494; 4096 worlds, two
+// steps and the readback 10.09 ms, now 9.76).
+constexpr uint32_t BATCH_STAGE = 512;  // bodies whose spheres are staged in shared memory
 __global__ void __launch_bounds__(256) k_batch_collide(BatchLaunch B) {
   __shared__ WorldScope s_scope;
+  __shared__ float4 s_sphere[BATCH_STAGE];
+  __shared__ uint8_t s_kind[BATCH_STAGE];  // 1: enabled, 2: dynamic
+  __shared__ uint2 s_queue[8][PAIR_QUEUE];
   const DWorld& w = s_scope.w;
   const StepParams& p = s_scope.p;
   for (;;) {
@@ -1729,23 +1737,62 @@ __global__ void __launch_bounds__(256) k_batch_collide(BatchLaunch B) {
       }
     }
     __syncthreads();
-    // every pair (i > j): triangular index k -> (i, j)
     const uint32_t n = p.n;
-    const uint32_t total = n * (n - 1u) / 2u;
-    for (uint32_t k = threadIdx.x; k < total; k += blockDim.x) {
-      uint32_t i = (uint32_t)((1.0f + sqrtf(1.0f + 8.0f * (float)k)) * 0.5f);
-      while (i * (i - 1u) / 2u > k) i--;
-      while ((i + 1u) * i / 2u <= k) i++;
-      uint32_t j = k - i * (i - 1u) / 2u;
-      if (!enabled(w, i) || !enabled(w, j)) continue;
-      bool di = w.size[i].w > 0.0f, dj = w.size[j].w > 0.0f;
-      if (!di && !dj) continue;
-      float4 pi4 = w.pos[i], pj4 = w.pos[j];
-      float3 dd = make_float3(pi4.x - pj4.x, pi4.y - pj4.y, pi4.z - pj4.z);
-      float r = w.moment[i].w + w.moment[j].w;
-      if (dot3(dd, dd) > r * r) continue;  // the sphere test: the same from either body's view
-      uint32_t pr = proberOf(w, p, i, j);
-      testPair(w, p, probeOf(w, pr), pr == i ? j : i);
+    if (n <= BATCH_STAGE) {
+      // every pair (i > j), a warp a row i, a lane a j: the sphere test from positions and radii in shared
+      // memory, the few that pass queued and given the full test on full warps
+      for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        const float4 x = w.pos[i];
+        s_sphere[i] = make_float4(x.x, x.y, x.z, w.moment[i].w);
+        s_kind[i] = uint8_t((enabled(w, i) ? 1u : 0u) | (w.size[i].w > 0.0f ? 2u : 0u));
+      }
+      __syncthreads();
+      const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+      uint2* Q = s_queue[warp];
+      uint32_t count = 0;
+      for (uint32_t i = 1u + warp; i < n; i += blockDim.x >> 5) {
+        const uint32_t ki = s_kind[i];
+        if (!(ki & 1u)) continue;
+        const float4 a = s_sphere[i];
+        for (uint32_t j0 = 0; j0 < i; j0 += 32u) {
+          const uint32_t j = j0 + lane;
+          bool push = false;
+          if (j < i) {
+            const uint32_t kj = s_kind[j];
+            const float4 b = s_sphere[j];
+            const float3 dd = make_float3(a.x - b.x, a.y - b.y, a.z - b.z);
+            const float r = a.w + b.w;
+            // the sphere test: the same from either body's view
+            push = (kj & 1u) && ((ki | kj) & 2u) && !(dot3(dd, dd) > r * r);
+          }
+          const uint32_t m = __ballot_sync(0xffffffffu, push);
+          if (m) {
+            if (push) Q[count + __popc(m & ((1u << lane) - 1u))] = make_uint2(i, j);
+            count += __popc(m);
+            __syncwarp();
+            if (count >= 32u) drainQueue(w, p, Q, count, lane);
+          }
+        }
+      }
+      while (count > 0u) drainQueue(w, p, Q, count, lane);
+    } else {
+      // every pair (i > j): triangular index k -> (i, j)
+      const uint32_t total = n * (n - 1u) / 2u;
+      for (uint32_t k = threadIdx.x; k < total; k += blockDim.x) {
+        uint32_t i = (uint32_t)((1.0f + sqrtf(1.0f + 8.0f * (float)k)) * 0.5f);
+        while (i * (i - 1u) / 2u > k) i--;
+        while ((i + 1u) * i / 2u <= k) i++;
+        uint32_t j = k - i * (i - 1u) / 2u;
+        if (!enabled(w, i) || !enabled(w, j)) continue;
+        bool di = w.size[i].w > 0.0f, dj = w.size[j].w > 0.0f;
+        if (!di && !dj) continue;
+        float4 pi4 = w.pos[i], pj4 = w.pos[j];
+        float3 dd = make_float3(pi4.x - pj4.x, pi4.y - pj4.y, pi4.z - pj4.z);
+        float r = w.moment[i].w + w.moment[j].w;
+        if (dot3(dd, dd) > r * r) continue;  // the sphere test: the same from either body's view
+        uint32_t pr = proberOf(w, p, i, j);
+        testPair(w, p, probeOf(w, pr), pr == i ? j : i);
+      }
     }
     __syncthreads();
     const uint32_t found = c[C_PAIRS];
