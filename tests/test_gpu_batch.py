@@ -5,7 +5,7 @@ import pytest
 
 import avbd_b200
 from avbd_b200 import BatchSolver3D, CudaSolver3D
-from avbd_b200.scenes import batched_worlds, cube_pyramid, demo_scene, drop_pile
+from avbd_b200.scenes import batched_worlds, cube_pyramid, demo_scene, drop_pile, small_world
 from oracle import Oracle
 from _util import cuda_from_oracle, oracle_sequential_colors, pose_diff
 
@@ -241,3 +241,27 @@ def test_batch_rejects_bad_worlds(cuda_lib):
     b.step(2)
     b.synchronize()
     b.destroy()
+
+
+@pytest.mark.parametrize('n', [1, 31, 40, 200, 513])
+def test_few_worlds_and_many_step_alike(cuda_lib, n):
+    """Up to as many worlds as SMs a world has a block of 512 threads, past that one of 256; worlds past
+    512 bodies test their pairs without staging. The same world in both, bit for bit, with its pairs."""
+    rng = np.random.default_rng(n)
+    scenes = [small_world(rng, n), small_world(rng, 20)]
+    few, many = avbd_b200.BatchSolver3D(2, 2 * (n + 30)), avbd_b200.BatchSolver3D(202, n + 30 + 202 * 25)
+    for b in (few, many):
+        b.set_params(scenes[0].params)
+        for s in scenes:
+            b.add_scene(s)
+    for _ in range(200):
+        many.add_scene(scenes[1])
+    for b in (few, many):
+        b.step(30)
+        b.synchronize()
+    for w in range(2):
+        assert few.read_bodies(w).tobytes() == many.read_bodies(w).tobytes()
+        a, c = few.read_counters(w), many.read_counters(w)
+        assert a == c and a['error'] == 0 and a['overflow'] == 0
+    few.destroy()
+    many.destroy()

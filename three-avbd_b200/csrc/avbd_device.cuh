@@ -295,7 +295,7 @@ __device__ inline void enterWorld(const BatchLaunch& B, uint32_t* queue, WorldSc
 #endif
 constexpr uint32_t BATCH_OVERFLOW = 1u, BATCH_NEAR_FULL = 2u;
 cudaError_t launch_batch_collision(const BatchLaunch& b, int blocks, int threads, cudaStream_t s);
-// worldThreads: 256, a block a world; 32, a warp a world (eight worlds a block)
+// worldThreads: 256 or 512, a block a world; 128, 64, 32: part of one (two, four, eight worlds a block)
 cudaError_t launch_batch_solve(const BatchLaunch& b, int blocks, int worldThreads, cudaStream_t s);
 int batch_collide_blocks_per_sm(int threads);
 int batch_solve_blocks_per_sm(int worldThreads);

@@ -24,6 +24,7 @@
 namespace avbd {
 
 constexpr int SOLVE_THREADS = 256;
+constexpr int WIDE_SOLVE_THREADS = 512;  // a block a world when there are no more worlds than SMs
 constexpr uint32_t ADJ_SORT_LOCAL = 24;  // adjacency lists up to this long are sorted in local memory
 constexpr long long BARRIER_CYCLES = 4000000000LL;  // about two seconds of SM clock
 
@@ -91,12 +92,12 @@ __device__ bool grid_sync(uint32_t* bar, uint32_t* counters) {
 
 // Exclusive scan of one block's range [lo, hi) in place; returns the range total (all threads).
 __device__ uint32_t block_scan_range(uint32_t* data, uint32_t lo, uint32_t hi) {
-  __shared__ uint32_t warpSums[SOLVE_THREADS / 32];
+  __shared__ uint32_t warpSums[WIDE_SOLVE_THREADS / 32];
   __shared__ uint32_t s_carry;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) s_carry = 0;
   __syncthreads();
-  for (uint32_t base = lo; base < hi; base += SOLVE_THREADS) {
+  for (uint32_t base = lo; base < hi; base += blockDim.x) {
     uint32_t i = base + threadIdx.x;
     uint32_t v = i < hi ? data[i] : 0u;
     uint32_t x = v;
@@ -108,8 +109,7 @@ __device__ uint32_t block_scan_range(uint32_t* data, uint32_t lo, uint32_t hi) {
     if (lane == 31) warpSums[warp] = x;
     __syncthreads();
     uint32_t before = 0, total = 0;
-#pragma unroll
-    for (int k = 0; k < SOLVE_THREADS / 32; k++) {
+    for (int k = 0; k < int(blockDim.x >> 5); k++) {
       uint32_t s = warpSums[k];
       if (k < warp) before += s;
       total += s;
@@ -184,7 +184,7 @@ struct BlockTeam {
   __device__ uint32_t lsize() const { return blockDim.x; }
   __device__ void lsync() const { __syncthreads(); }
   __device__ uint32_t scan(uint32_t* data, uint32_t lo, uint32_t hi) const { return block_scan_range(data, lo, hi); }
-  __device__ uint32_t laneBudget() const { return size(); }
+  __device__ uint32_t laneBudget() const { return SOLVE_THREADS; }
 };
 // Exclusive scan of a sub-block team's range [lo, hi) in place (kT threads, two or four warps, synced
 // by named barrier 1 + unit); returns the range total (all threads).
@@ -1733,8 +1733,10 @@ __global__ void __launch_bounds__(SOLVE_THREADS, kBlocksPerSm) k_topology_solve(
 }
 
 // Batched worlds: each block takes worlds from the queue (largest first) and runs the same
-// topology + solve code for one world at block scope.
-__global__ void __launch_bounds__(SOLVE_THREADS, 2) k_batch_solve(BatchLaunch B) {
+// topology + solve code for one world at block scope. Lane classes are sized for SOLVE_THREADS at either
+// block size, so the results are the same bit for bit.
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, 512 / kThreads) k_batch_solve(BatchLaunch B) {
   __shared__ WorldScope s_scope;
   const WorldScope& S = s_scope;
   const DWorld& w = S.w;
@@ -1744,11 +1746,11 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 2) k_batch_solve(BatchLaunch B)
     if (threadIdx.x == 0) enterWorld(B, &B.queue[1], s_scope);
     __syncthreads();
     if (S.world >= B.nWorlds) return;
-    for (uint32_t i = threadIdx.x; i <= p.n; i += SOLVE_THREADS) {
+    for (uint32_t i = threadIdx.x; i <= p.n; i += kThreads) {
       w.adjStart[i] = 0u;
       w.adjFill[i] = 0u;
     }
-    for (uint32_t k = threadIdx.x; k < (uint32_t)BUCKET_WORDS; k += SOLVE_THREADS) w.bucket[k] = 0u;
+    for (uint32_t k = threadIdx.x; k < (uint32_t)BUCKET_WORDS; k += kThreads) w.bucket[k] = 0u;
     __syncthreads();
     BlockTeam team;
     topologySolve(w, p, team);
@@ -1793,7 +1795,7 @@ int batch_solve_blocks_per_sm(int worldThreads) {
   if (worldThreads == 32) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_batch_solve_sub<32>, SOLVE_THREADS, 0);
   else if (worldThreads == 64) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_batch_solve_sub<64>, SOLVE_THREADS, 0);
   else if (worldThreads == 128) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_batch_solve_sub<128>, SOLVE_THREADS, 0);
-  else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_batch_solve, SOLVE_THREADS, 0);
+  else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_batch_solve<SOLVE_THREADS>, SOLVE_THREADS, 0);
   return perSm;
 }
 
@@ -1801,7 +1803,8 @@ cudaError_t launch_batch_solve(const BatchLaunch& b, int blocks, int worldThread
   if (worldThreads == 32) k_batch_solve_sub<32><<<blocks, SOLVE_THREADS, 0, s>>>(b);
   else if (worldThreads == 64) k_batch_solve_sub<64><<<blocks, SOLVE_THREADS, 0, s>>>(b);
   else if (worldThreads == 128) k_batch_solve_sub<128><<<blocks, SOLVE_THREADS, 0, s>>>(b);
-  else k_batch_solve<<<blocks, SOLVE_THREADS, 0, s>>>(b);
+  else if (worldThreads == WIDE_SOLVE_THREADS) k_batch_solve<WIDE_SOLVE_THREADS><<<blocks, WIDE_SOLVE_THREADS, 0, s>>>(b);
+  else k_batch_solve<SOLVE_THREADS><<<blocks, SOLVE_THREADS, 0, s>>>(b);
   return cudaGetLastError();
 }
 
