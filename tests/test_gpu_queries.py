@@ -153,7 +153,7 @@ def test_raycast_matches_oracle(cuda_lib):
     w.destroy()
 
 
-@pytest.mark.parametrize('n, rays', [(1, 1), (255, 63), (300, 65), (1100, 4800)])
+@pytest.mark.parametrize('n, rays', [(1, 1), (31, 9), (255, 63), (1022, 65), (1023, 40), (1024, 40), (1100, 4800)])
 def test_raycast_tiles_and_far_origins(cuda_lib, n, rays):
     """Rays at the edges of the ray and body tiles, from near and from 2 km away, on long, flat and
     unnormalised bodies: all in one call as in calls of 32, and a sample of the distances against the

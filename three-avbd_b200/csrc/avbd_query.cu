@@ -242,13 +242,10 @@ __device__ float rayTrace(const DWorld& w, uint32_t b, const DRay& r, float3& n)
   return t <= 0.0f ? 0.0f : t;  // never -0: its bits would order as a huge distance
 }
 
-// Per body a sphere that holds every point rayTrace can hit, xyz and squared radius: -inf for a body
-// the query skips, +inf (always traced) for a hull, whose planes are not bounded by a record field,
-// and for a rotation that is not of unit length, which would stretch the body. Resets the keys too.
-__global__ void k_ray_prepare(DWorld w, RayLaunch R) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < R.n) R.best[i] = NO_HIT;
-  if (i >= R.bodies) return;
+// A sphere that holds every point of body i that rayTrace can hit, xyz and squared radius: -inf for a
+// body the query skips, +inf (always traced) for a hull, whose planes are not bounded by a record field,
+// and for a rotation that is not of unit length, which would stretch the body.
+__device__ __forceinline__ float4 raySphere(const DWorld& w, const RayLaunch& R, uint32_t i) {
   const float4 pos = w.pos[i], size = w.size[i], q = w.rot[i];
   const float shape = w.avel[i].w;
   const float inf = __int_as_float(0x7f800000);
@@ -257,74 +254,34 @@ __global__ void k_ray_prepare(DWorld w, RayLaunch R) {
   else if (shape > 2.5f) r2 = inf;
   if (!(fabsf(q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w - 1.0f) < 1e-3f)) r2 = inf;
   if (rayIgnores(w, R, i)) r2 = -inf;
-  R.bounds[i] = make_float4(pos.x, pos.y, pos.z, r2);
+  return make_float4(pos.x, pos.y, pos.z, r2);
+}
+// Whether a ray passes sphere x (w: its squared radius, grown): the squared distance of the centre from
+// the ray, or from its origin where the centre lies behind. The comparison is negated and the maximum keeps
+// a NaN, so that a pair with a NaN in it is traced.
+__device__ __forceinline__ bool nearSphere(float4 x, float3 o, float3 d) {
+  const float3 rel = f3(x) - o;
+  const float along = dot3(rel, d), far2 = dot3(rel, rel);
+  float ahead;
+  asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(ahead) : "f"(along));
+  return !(far2 - ahead * ahead > x.w + 8.0e-6f * far2);
+}
+// Every body's sphere, once for all the blocks that read it; resets the keys too
+__global__ void k_ray_prepare(DWorld w, RayLaunch R) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < R.n) R.best[i] = NO_HIT;
+  if (i < R.bodies) R.bounds[i] = raySphere(w, R, i);
 }
 
-// A tile of rays (blockIdx.y) against a block of bodies, kBodies of them a thread. A ray is traced
-// against a body only where it passes the body's sphere, grown by 4e-6 of the squared distance from the
-// origin (over thirty f32 roundings of it: rayTrace's own rounding, its sphere discriminant's above all)
-// so that no hit that rayTrace would report is passed over: tracing every ray against every body read
-// 64 bytes and ran six plane divisions for each pair, and one pair in a thousand hits (4096 rays into
-// 20000 bodies: 1478 us a call, now 341). What is left is the sphere test, bound by instruction issue:
-// the rays stay in shared memory and each is read once for kBodies tests. The least (distance bits, body) key is the nearest hit and, among hits at the same
-// distance, the lowest body index, as the reference's two atomic passes find it; keys meet in shared
-// memory and each block ends with one global atomic a ray that hit something.
-constexpr uint32_t RAY_THREADS = 256, RAY_TILE = 64;
-template <int kBodies>
-__global__ void __launch_bounds__(RAY_THREADS) k_ray_nearest(DWorld w, RayLaunch R) {
-  __shared__ DRay s_ray[RAY_TILE];
-  __shared__ unsigned long long s_best[RAY_TILE];
-  const uint32_t r0 = blockIdx.y * RAY_TILE, rays = min(RAY_TILE, R.n - r0);
-  if (threadIdx.x < rays) {
-    s_ray[threadIdx.x] = R.rays[r0 + threadIdx.x];
-    s_best[threadIdx.x] = NO_HIT;
-  }
-  float4 body[kBodies];
-  const uint32_t b0 = blockIdx.x * (RAY_THREADS * kBodies) + threadIdx.x;
-#pragma unroll
-  for (int k = 0; k < kBodies; k++) {
-    const uint32_t b = b0 + k * RAY_THREADS;
-    body[k] = b < R.bodies ? R.bounds[b] : make_float4(0.0f, 0.0f, 0.0f, -__int_as_float(0x7f800000));
-  }
-  __syncthreads();
-  for (uint32_t r = 0; r < rays; r++) {
-    const float4 o = s_ray[r].o, d = s_ray[r].d;
-    uint32_t pass = 0;
-#pragma unroll
-    for (int k = 0; k < kBodies; k++) {
-      const float3 rel = f3(body[k]) - f3(o);
-      const float along = dot3(rel, f3(d)), far2 = dot3(rel, rel);
-      const float3 off = rel - f3(d) * along;
-      const float limit = body[k].w * 1.0001f + 4.0e-6f * far2;
-      // negated, so that a comparison with NaN traces the body
-      if (!(dot3(off, off) > limit) && !(along < 0.0f && far2 > limit)) pass |= 1u << k;
-    }
-    while (pass) {
-      const uint32_t b = b0 + (__ffs(pass) - 1) * RAY_THREADS;
-      pass &= pass - 1u;
-      if (b >= R.bodies || rayIgnores(w, R, b)) continue;
-      float3 n;
-      const float t = rayTrace(w, b, s_ray[r], n);
-      if (t >= 0.0f) atomicMin(&s_best[r], ((unsigned long long)__float_as_uint(t) << 32) | b);
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x < rays && s_best[threadIdx.x] != NO_HIT) atomicMin(R.best + r0 + threadIdx.x, s_best[threadIdx.x]);
-}
-
-// Per ray: the nearest hit's record, its normal in world axes (raycast.ts finish), as avbd_ray_hit's
-// eight words. The point's products and sums round one by one.
-__global__ void k_ray_finish(DWorld w, RayLaunch R) {
-  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= R.n) return;
-  const unsigned long long key = R.best[r];
+// Ray r's hit from its nearest key: the record's eight words, the normal in world axes (raycast.ts
+// finish). The point's products and sums round one by one.
+__device__ __forceinline__ void finishRay(const DWorld& w, const RayLaunch& R, uint32_t r, const DRay& ray, unsigned long long key) {
   if (key == NO_HIT) {
     R.hits[2 * r] = make_float4(__uint_as_float(0xffffffffu), -1.0f, 0.0f, 0.0f);
     R.hits[2 * r + 1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     return;
   }
   const uint32_t b = uint32_t(key);
-  const DRay ray = R.rays[r];
   float3 n;
   const float t = rayTrace(w, b, ray, n);
   float3 wn = qrotate(w.rot[b], n);
@@ -332,6 +289,96 @@ __global__ void k_ray_finish(DWorld w, RayLaunch R) {
   const float px = __fadd_rn(ray.o.x, __fmul_rn(ray.d.x, t)), py = __fadd_rn(ray.o.y, __fmul_rn(ray.d.y, t)), pz = __fadd_rn(ray.o.z, __fmul_rn(ray.d.z, t));
   R.hits[2 * r] = make_float4(__uint_as_float(b), t, px, py);
   R.hits[2 * r + 1] = make_float4(pz, wn.x, wn.y, wn.z);
+}
+
+// A tile of rays (blockIdx.y) against a chunk of bodies, whose spheres are staged in shared memory: a warp
+// takes a ray and its lanes the spheres. A ray is traced against a body only where it passes the body's
+// sphere, grown by 8e-6 of the squared distance from the origin (over sixty f32 roundings of it: the
+// test's own, which come to thirteen, and rayTrace's, its sphere discriminant's above all) so that no hit
+// that rayTrace would report is passed over; the pairs that pass are queued and traced a lane each. Tracing every ray against every
+// body read 64 bytes and ran six plane divisions for each pair, and one pair in a thousand hits; tracing
+// where the sphere test passed, a lane or two at a time, left few rays waiting on one trace after another.
+// The sphere test is bound by instruction issue. The least (distance bits, body) key is the nearest hit
+// and, among hits at the same distance, the lowest body index, as the reference's two atomic passes find
+// it; keys meet in shared memory and each block ends with one global atomic a ray that hit something.
+// kSpheres: a block makes its bodies' spheres itself instead of reading what k_ray_prepare laid out once;
+// kFinish: it holds every body and finishes its rays. So a query of up to RAY_CHUNK bodies is one launch and
+// one of few rays needs no preparing pass. Microseconds a call before and after, 4096 rays into 20000
+// bodies: 1476, 232; 1000 into 3000: 122, 79; 100 into 50: 48, 47; 1 into 50: 41, 41.
+constexpr uint32_t RAY_THREADS = 256, RAY_WARPS = RAY_THREADS / 32, RAY_TILE = 64, RAY_CHUNK = 1024;
+template <bool kSpheres, bool kFinish>
+__global__ void __launch_bounds__(RAY_THREADS) k_ray_nearest(DWorld w, RayLaunch R, uint32_t tile, uint32_t chunk) {
+  __shared__ DRay s_ray[RAY_TILE];
+  __shared__ unsigned long long s_best[RAY_TILE];
+  __shared__ float4 s_sphere[RAY_CHUNK];
+  __shared__ uint32_t s_queue[RAY_WARPS][64];  // ray of the tile << 16 | body of the chunk
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const uint32_t r0 = blockIdx.y * tile, rays = min(tile, R.n - r0);
+  const uint32_t b0 = blockIdx.x * chunk, bodies = min(chunk, R.bodies - b0);
+  if (threadIdx.x < rays) {
+    s_ray[threadIdx.x] = R.rays[r0 + threadIdx.x];
+    s_best[threadIdx.x] = NO_HIT;
+  }
+  for (uint32_t b = threadIdx.x; b < bodies; b += RAY_THREADS) {
+    float4 x = kSpheres ? raySphere(w, R, b0 + b) : R.bounds[b0 + b];
+    x.w *= 1.0001f;
+    s_sphere[b] = x;
+  }
+  __syncthreads();
+  uint32_t* Q = s_queue[warp];
+  uint32_t count = 0;
+  auto drain = [&]() {
+    const uint32_t take = min(count, 32u);
+    const uint32_t e = lane < take ? Q[lane] : 0u;
+    __syncwarp();
+    if (lane + take < count) Q[lane] = Q[lane + take];
+    __syncwarp();
+    count -= take;
+    if (lane >= take) return;
+    const uint32_t r = e >> 16, b = b0 + (e & 0xffffu);
+    if (rayIgnores(w, R, b)) return;
+    float3 n;
+    const float t = rayTrace(w, b, s_ray[r], n);
+    if (t >= 0.0f) atomicMin(&s_best[r], ((unsigned long long)__float_as_uint(t) << 32) | b);
+  };
+  auto push = [&](bool pass, uint32_t r, uint32_t b) {
+    const uint32_t m = __ballot_sync(0xffffffffu, pass);
+    if (!m) return;
+    if (pass) Q[count + __popc(m & ((1u << lane) - 1u))] = (r << 16) | b;
+    count += __popc(m);
+    __syncwarp();
+    if (count >= 32u) drain();
+  };
+  // two rays at a time where there are more than warps, so that a sphere is read once for both
+  const uint32_t step = rays > RAY_WARPS ? 2u : 1u;
+  for (uint32_t r = warp * step; r < rays; r += RAY_WARPS * step) {
+    const uint32_t r2 = r + 1u < rays ? r + 1u : r;
+    const bool two = step == 2u && r2 != r;
+    const float3 o = f3(s_ray[r].o), d = f3(s_ray[r].d), o2 = f3(s_ray[r2].o), d2 = f3(s_ray[r2].d);
+    for (uint32_t c = 0; c < bodies; c += 32u) {
+      const uint32_t b = c + lane;
+      bool pass = false, pass2 = false;
+      if (b < bodies) {
+        const float4 x = s_sphere[b];
+        pass = nearSphere(x, o, d);
+        if (two) pass2 = nearSphere(x, o2, d2);
+      }
+      if (!__any_sync(0xffffffffu, pass || pass2)) continue;
+      push(pass, r, b);
+      push(pass2, r2, b);
+    }
+  }
+  while (count > 0u) drain();
+  __syncthreads();
+  if (threadIdx.x >= rays) return;
+  const unsigned long long key = s_best[threadIdx.x];
+  if (kFinish) finishRay(w, R, r0 + threadIdx.x, s_ray[threadIdx.x], key);
+  else if (key != NO_HIT) atomicMin(R.best + r0 + threadIdx.x, key);
+}
+
+__global__ void k_ray_finish(DWorld w, RayLaunch R) {
+  const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r < R.n) finishRay(w, R, r, R.rays[r], R.best[r]);
 }
 static_assert(sizeof(avbd_ray_hit) == 2 * sizeof(float4) && offsetof(avbd_ray_hit, point) == 8 && offsetof(avbd_ray_hit, normal) == 20, "a hit is eight words");
 
@@ -560,13 +607,29 @@ int avbd_raycast(avbd_world* w, const avbd_ray* rays, uint32_t n, const uint32_t
     R.nIgnore = n_ignore;
     R.mask = mask;
     for (uint32_t k = 0; k < n_ignore; k++) R.ignore[k] = ignore[k];
-    const uint32_t tiles = grid_for(n, RAY_TILE);
-    k_ray_prepare<<<grid_for(std::max(n, w->n), 256), 256, 0, w->stream>>>(w->d, R);
-    // four bodies a thread once that still fills the SMs
-    if (grid_for(w->n, 4 * RAY_THREADS) * tiles >= 148u) k_ray_nearest<4><<<dim3(grid_for(w->n, 4 * RAY_THREADS), tiles), RAY_THREADS, 0, w->stream>>>(w->d, R);
-    else if (w->n) k_ray_nearest<1><<<dim3(grid_for(w->n, RAY_THREADS), tiles), RAY_THREADS, 0, w->stream>>>(w->d, R);
-    k_ray_finish<<<grid_for(n, 128), 128, 0, w->stream>>>(w->d, R);
-    e = cudaGetLastError();
+    // rays a block: enough blocks for two an SM, a warp a ray at the least; still too few blocks: a quarter
+    // of the bodies each
+    uint32_t chunk = RAY_CHUNK, chunks = std::max(1u, grid_for(w->n, chunk));
+    const uint32_t tile = std::min(RAY_TILE, std::max(RAY_WARPS, grid_for(uint32_t(uint64_t(n) * chunks / 296u), RAY_WARPS) * RAY_WARPS));
+    const uint32_t tiles = grid_for(n, tile);
+    if (chunks > 1u && chunks * tiles < 296u) {
+      chunk = RAY_CHUNK / 4u;
+      chunks = grid_for(w->n, chunk);
+    }
+    const dim3 grid(chunks, tiles);
+    if (chunks == 1u) {
+      k_ray_nearest<true, true><<<grid, RAY_THREADS, 0, w->stream>>>(w->d, R, tile, chunk);
+    } else {
+      if (tiles <= 32u) {
+        e = cudaMemsetAsync(w->rayBest, 0xff, n * sizeof(unsigned long long), w->stream);
+        k_ray_nearest<true, false><<<grid, RAY_THREADS, 0, w->stream>>>(w->d, R, tile, chunk);
+      } else {
+        k_ray_prepare<<<grid_for(std::max(n, w->n), 256), 256, 0, w->stream>>>(w->d, R);
+        k_ray_nearest<false, false><<<grid, RAY_THREADS, 0, w->stream>>>(w->d, R, tile, chunk);
+      }
+      k_ray_finish<<<grid_for(n, 128), 128, 0, w->stream>>>(w->d, R);
+    }
+    if (e == cudaSuccess) e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemcpyAsync(hits, w->rayHits, n * sizeof(avbd_ray_hit), cudaMemcpyDeviceToHost, w->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(w->stream);
