@@ -288,8 +288,8 @@ cudaError_t enqueueStep(avbd_batch* b, const BatchLaunch& L) {
   cudaMemsetAsync(b->dQueue, 0, 2 * sizeof(uint32_t), b->stream);
   cudaMemsetAsync(b->dStatus, 0, 2 * sizeof(uint32_t), b->stream);
   // No more worlds than SMs, a block each: the step lasts as long as its largest world, and the SM's other
-  // half would stand empty, so a world gets 512 threads. (96 worlds of
-  // 16 to 250 bodies, one step and the readback: 494 us, now 387.)
+  // half would stand empty, so a world gets 512 threads. (96 worlds of 16 to 250 bodies, one step and the
+  // readback: 494 us, now 387.)
   const bool wide = int(L.nWorlds) <= b->sms && b->solveBlocks >= int(L.nWorlds) && b->worldThreads == BATCH_SOLVE_THREADS;
   cudaError_t e = launch_batch_collision(L, b->collideBlocks, wide ? 512 : b->collideThreads, b->stream);
   if (e != cudaSuccess) return e;

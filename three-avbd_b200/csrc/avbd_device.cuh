@@ -31,6 +31,7 @@ constexpr float REUSE_LIN_TOL = 0.002f, REUSE_ANG_TOL = 0.002f;  // gpu/layout.t
 constexpr float REST_SPEED = 0.1f;
 constexpr float NEAREST_FRACTION = 0.05f;
 constexpr uint32_t OWNER_BIT = 0x80000000u;  // incidence entry: this body updates the constraint's dual
+constexpr uint32_t BODY_WORDS = 4, WORD_GROUP = 8;  // the dataflow sweep's words a body, and bodies whose words are interleaved
 // incidence partner word: index | PARTNER_DYNAMIC | PARTNER_EARLIER (its colour comes first in the sweep)
 constexpr uint32_t PARTNER_DYNAMIC = 0x80000000u, PARTNER_EARLIER = 0x40000000u, PARTNER_MASK = 0x3fffffffu;
 constexpr int LANE_CLASSES = 6;                // 1, 2, 4, 8, 16, 32 lanes per body
@@ -110,14 +111,15 @@ struct DWorld {
   uint32_t *incCount, *incStart;
   uint2* incList;         // per incidence: constraint row (joint slot, or nj + point slot) | OWNER_BIT, partner word
   float2* c0t;            // per point slot: C0 along t1 and t2, whose place in the point's record the dataflow sweep's tags take (null: batched worlds)
-  float4* words;          // per body: the dataflow sweep's four tagged words (its pose since x-)
+  float4* words;          // per body: the dataflow sweep's four tagged words (its pose since x-), in groups of eight bodies
   uint32_t* done;         // per body: iterations after which the joints it updates are written
   uint4* laneTable;       // per lane of the dataflow sweep: body, first row, row end, L | sub << 8
   uint32_t* bucket;       // BUCKET_WORDS: counts, starts (+ total), fill cursors, lane bases, lane totals per colour
   // Per body, the step's unknowns relative to x- (kept by the solve, precise at any distance from the
   // origin, where an absolute f32 position rounds to its magnitude's ulp): dlin = x - x- and
   // dang = (2 vec(r), r.w) with r the rotation since x- (q = r q-, so qsub(q, q-) = dang.xyz); and
-  // the inertial target y the same way: ylin = y - x-, yang = the rotation from q- to y's rotation. The dataflow sweep keeps its poses in `words` instead of dlin and dang.
+  // the inertial target y the same way: ylin = y - x-, yang = the rotation from q- to y's rotation. The
+  // dataflow sweep keeps its poses in `words` instead of dlin and dang.
   float4 *dlin, *dang, *ylin, *yang;
   // contact reuse (wgsl-collision.ts:20-44): per body its reference pose (zero rotation: none yet);
   // the step it last moved past the tolerances is kept in ypos.w (the record's moved_step word)

@@ -471,7 +471,7 @@ int avbd_world_create(const avbd_config* cfg, avbd_world** out) {
   A(dalloc(w, &d.refPos, B));
   A(dalloc(w, &d.refRot, B));
   A(dalloc(w, &d.done, B));
-  A(dalloc(w, &d.words, size_t(B) * 4));
+  A(dalloc(w, &d.words, (size_t(B) + WORD_GROUP - 1) / WORD_GROUP * WORD_GROUP * 4));
   A(dalloc(w, &d.scanScratch, w->maxSolveBlocks + 1));
   A(dalloc(w, &d.counters, COUNTER_WORDS));
   A(dalloc(w, &d.barrier, 2));

@@ -799,14 +799,21 @@ __device__ __forceinline__ uint32_t tagOf(float4 v) { return __float_as_uint(v.w
 // assembler narrows the access to several smaller ones, and a tag could arrive with an older value.
 __device__ __forceinline__ bool brokenWord(float4 v) { return (__float_as_uint(v.y) & __float_as_uint(v.z)) == 0xffffffffu; }
 
-// A body's four words: displacement | 2 vec r | rotation x y z | rotation w, r's w, a filler
-constexpr int BODY_WORDS = 4;
+// A body's four words: displacement | 2 vec r | rotation x y z | rotation w, r's w, a filler. Eight bodies'
+// first words lie together, then their second ones and so on: bodies that are near one another in number
+// are often solved and read by one warp, whose accesses to a word then share lines, and a body's words
+// are at fixed distances. With a body's words side by side a warp's load touched a sector a lane, half of
+// it for another load (microseconds a solve: 100000 bodies 1175, now 1142; 20000 371, 364; 200 heaped
+// chains of 50 370, 360; 1000 hanging ones 382, 328; groups of 4 in between, of 32 equal to 8).
+__device__ __forceinline__ float4* bodyWords(const DWorld& w, uint32_t i) {
+  return w.words + size_t(i / WORD_GROUP) * (BODY_WORDS * WORD_GROUP) + i % WORD_GROUP;
+}
 __device__ __forceinline__ void stBody(const DWorld& w, uint32_t i, float3 dl, float4 dang, float4 q, uint32_t tag) {
-  float4* b = w.words + size_t(i) * BODY_WORDS;
+  float4* b = bodyWords(w, i);
   stWord(b, dl.x, dl.y, dl.z, tag);
-  stWord(b + 1, dang.x, dang.y, dang.z, tag);
-  stWord(b + 2, q.x, q.y, q.z, tag);
-  stWord(b + 3, q.w, dang.w, dl.x, tag);
+  stWord(b + WORD_GROUP, dang.x, dang.y, dang.z, tag);
+  stWord(b + 2 * WORD_GROUP, q.x, q.y, q.z, tag);
+  stWord(b + 3 * WORD_GROUP, q.w, dang.w, dl.x, tag);
 }
 
 // Keeps a waiting lane's polls bounded: false past the clock budget, or once any wait of the launch
@@ -830,14 +837,6 @@ struct PollLimit {
     return true;
   }
 };
-// Waits until a body's joint count (published with release semantics) reaches `need`
-__device__ inline bool waitDone(const DWorld& w, const uint32_t* flag, uint32_t need) {
-  PollLimit limit;
-  while (ld_acquire_gpu(flag) < need)
-    if (!limit.again(w)) return false;
-  return true;
-}
-
 __device__ __forceinline__ void st_release_gpu(uint32_t* p, uint32_t v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -1018,11 +1017,11 @@ struct FlowRow {
 __device__ __forceinline__ void issueRow(const DWorld& w, const StepParams& p, uint2 inc, FlowRow& f) {
   const uint32_t cs = (inc.x & ~OWNER_BIT) - p.nj;
   const float4* pt = w.cPt[p.cur] + 4 * size_t(cs);
-  const float4* b = w.words + size_t(inc.y & PARTNER_MASK) * BODY_WORDS;
+  const float4* b = bodyWords(w, inc.y & PARTNER_MASK);
   f.b0 = ldWord(b);
-  f.b1 = ldWord(b + 1);
-  f.b2 = ldWord(b + 2);
-  f.b3 = ldWord(b + 3);
+  f.b1 = ldWord(b + WORD_GROUP);
+  f.b2 = ldWord(b + 2 * WORD_GROUP);
+  f.b3 = ldWord(b + 3 * WORD_GROUP);
   f.pen = ldWord(pt + K_PEN);
   f.lam = ldWord(pt + K_LAM);
   f.ra = pt[K_RA];
@@ -1041,7 +1040,7 @@ __device__ __forceinline__ uint32_t needPose(uint32_t partnerWord, uint32_t it) 
 __device__ __forceinline__ bool settleRow(const DWorld& w, const StepParams& p, uint2 inc, uint32_t it, FlowRow& f) {
   const uint32_t need = needPose(inc.y, it), needRow = (inc.x & OWNER_BIT) ? 0u : it;
   const float4* pt = w.cPt[p.cur] + 4 * size_t((inc.x & ~OWNER_BIT) - p.nj);
-  const float4* b = w.words + size_t(inc.y & PARTNER_MASK) * BODY_WORDS;
+  const float4* b = bodyWords(w, inc.y & PARTNER_MASK);
   PollLimit limit;
   for (;;) {
     const bool m0 = tagOf(f.b0) < need, m1 = tagOf(f.b1) < need, m2 = tagOf(f.b2) < need, m3 = tagOf(f.b3) < need || brokenWord(f.b3);
@@ -1049,9 +1048,9 @@ __device__ __forceinline__ bool settleRow(const DWorld& w, const StepParams& p, 
     if (!(m0 | m1 | m2 | m3 | mp | ml)) return true;
     if (!limit.again(w)) return false;
     if (m0) f.b0 = ldWord(b);
-    if (m1) f.b1 = ldWord(b + 1);
-    if (m2) f.b2 = ldWord(b + 2);
-    if (m3) f.b3 = ldWord(b + 3);
+    if (m1) f.b1 = ldWord(b + WORD_GROUP);
+    if (m2) f.b2 = ldWord(b + 2 * WORD_GROUP);
+    if (m3) f.b3 = ldWord(b + 3 * WORD_GROUP);
     if (mp) f.pen = ldWord(pt + K_PEN);
     if (ml) f.lam = ldWord(pt + K_LAM);
   }
@@ -1074,26 +1073,34 @@ __device__ __forceinline__ void flowPoint(const DWorld& w, uint2 inc, uint32_t b
   v.other = wordPose(f.b0, f.b1, f.b2, f.b3);
   viewPoint(w, f.geo, body, inc.y & PARTNER_MASK, v);
 }
-// A joint's partner (its words polled) and, when the partner updates the joint, that update awaited
+// A joint's partner (its words polled) and, when the partner updates the joint, that update awaited. All
+// five loads are in flight together; the count comes last, so that its acquire orders the joint's record.
+// (One wait after another: 4000 heaped hulls on 200 chains 20 us a solve longer.)
 constexpr uint32_t WORLD_PARTNER = 0x7fffffffu & PARTNER_MASK;  // a world joint's other end
 __device__ inline bool flowJoint(const DWorld& w, uint2 inc, uint32_t it, Pose& P) {
   const uint32_t partner = inc.y & PARTNER_MASK;
   if (partner == WORLD_PARTNER) return true;
-  const uint32_t need = needPose(inc.y, it);
-  const float4* b = w.words + size_t(partner) * BODY_WORDS;
-  float4 v[BODY_WORDS];
+  const uint32_t need = needPose(inc.y, it), needCount = (inc.x & OWNER_BIT) ? 0u : it;
+  const float4* b = bodyWords(w, partner);
+  float4 b0 = ldWord(b), b1 = ldWord(b + WORD_GROUP), b2 = ldWord(b + 2 * WORD_GROUP), b3 = ldWord(b + 3 * WORD_GROUP);
+  const float3 x0 = f3(w.ipos[partner]);
+  uint32_t count = needCount ? ld_acquire_gpu(w.done + partner) : 0u;
   PollLimit limit;
-#pragma unroll
-  for (int k = 0; k < BODY_WORDS; k++) {
-    v[k] = ldWord(b + k);
-    while (tagOf(v[k]) < need || brokenWord(v[k])) {
-      if (!limit.again(w)) return false;
-      v[k] = ldWord(b + k);
-    }
+  for (;;) {
+    const bool m0 = tagOf(b0) < need || brokenWord(b0), m1 = tagOf(b1) < need || brokenWord(b1);
+    const bool m2 = tagOf(b2) < need || brokenWord(b2), m3 = tagOf(b3) < need || brokenWord(b3);
+    const bool mc = count < needCount;
+    if (!(m0 | m1 | m2 | m3 | mc)) break;
+    if (!limit.again(w)) return false;
+    if (m0) b0 = ldWord(b);
+    if (m1) b1 = ldWord(b + WORD_GROUP);
+    if (m2) b2 = ldWord(b + 2 * WORD_GROUP);
+    if (m3) b3 = ldWord(b + 3 * WORD_GROUP);
+    if (mc) count = ld_acquire_gpu(w.done + partner);
   }
-  P = wordPose(v[0], v[1], v[2], v[3]);
-  P.x0 = f3(w.ipos[partner]);
-  return (inc.x & OWNER_BIT) || it == 0u || waitDone(w, w.done + partner, it);
+  P = wordPose(b0, b1, b2, b3);
+  P.x0 = x0;
+  return true;
 }
 
 // One 32-lane chunk of the dataflow sweep, solveLanes with every word awaited (above) and written with
@@ -1109,8 +1116,8 @@ __device__ __forceinline__ bool flowLanes(const DWorld& w, const StepParams& p, 
   accZero(acc);
   bool ok = true, joints = false;
   if (active) {
-    const float4* b = w.words + size_t(body) * BODY_WORDS;
-    own = wordPose(ldWord(b), ldWord(b + 1), ldWord(b + 2), ldWord(b + 3));
+    const float4* b = bodyWords(w, body);
+    own = wordPose(ldWord(b), ldWord(b + WORD_GROUP), ldWord(b + 2 * WORD_GROUP), ldWord(b + 3 * WORD_GROUP));
     own.q0 = w.irot[body];
     if (p.nj) own.x0 = f3(w.ipos[body]);
     if (sub == 0) addInertia(acc, w, body, own, dt2);
@@ -1694,11 +1701,11 @@ __device__ void topologySolve(const DWorld& w, const StepParams& p, Team& team) 
       // x = x- + the displacement (the sweep keeps only the displacement, which partners read)
       float3 dl, dang;
       if constexpr (Team::kDataflow) {
-        const float4* b = w.words + size_t(i) * BODY_WORDS;
-        const float4 b2 = ldWord(b + 2);
+        const float4* b = bodyWords(w, i);
+        const float4 b2 = ldWord(b + 2 * WORD_GROUP);
         dl = f3(ldWord(b));
-        dang = f3(ldWord(b + 1));
-        w.rot[i] = make_float4(b2.x, b2.y, b2.z, ldWord(b + 3).x);
+        dang = f3(ldWord(b + WORD_GROUP));
+        w.rot[i] = make_float4(b2.x, b2.y, b2.z, ldWord(b + 3 * WORD_GROUP).x);
       } else {
         dl = f3(w.dlin[i]);
         dang = f3(w.dang[i]);
