@@ -148,7 +148,7 @@ struct DRay {
   float4 d;  // unit direction
 };
 struct RayLaunch {
-  const DRay* rays;
+  const DRay* rays;          // as the caller gave them: loadRay normalises
   unsigned long long* best;  // per ray: distance bits << 32 | body (all ones: no hit)
   float4* hits;              // per ray: its avbd_ray_hit record
   float4* bounds;            // per body: centre, squared radius of the sphere around it
@@ -156,6 +156,20 @@ struct RayLaunch {
   uint32_t ignore[AVBD_RAY_MAX_IGNORED];
 };
 constexpr unsigned long long NO_HIT = ~0ull;
+
+// Ray i, its direction normalised in double (raycast.ts:193-196; a zero one stays zero), rounded as the
+// host's arithmetic would round it. On the host, with the records that it filled, this was a tenth of a
+// call of many rays (microseconds a call with it there and here: 4096 rays into 50 bodies 136, 120; into
+// 20000 234, 223).
+__device__ __forceinline__ DRay loadRay(const RayLaunch& R, uint32_t i) {
+  DRay r = R.rays[i];
+  const double x = r.d.x, y = r.d.y, z = r.d.z;
+  double l = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z)));
+  if (!(l > 0.0)) l = 1.0;
+  r.o.w = r.o.w > 3.0e38f ? 3.0e38f : r.o.w;
+  r.d = make_float4(__double2float_rn(__ddiv_rn(x, l)), __double2float_rn(__ddiv_rn(y, l)), __double2float_rn(__ddiv_rn(z, l)), 0.0f);
+  return r;
+}
 
 __device__ __forceinline__ bool rayIgnores(const DWorld& w, const RayLaunch& R, uint32_t b) {
   if (bodyDisabled(w, b)) return true;
@@ -304,7 +318,7 @@ __device__ __forceinline__ void finishRay(const DWorld& w, const RayLaunch& R, u
 // kSpheres: a block makes its bodies' spheres itself instead of reading what k_ray_prepare laid out once;
 // kFinish: it holds every body and finishes its rays. So a query of up to RAY_CHUNK bodies is one launch and
 // one of few rays needs no preparing pass. Microseconds a call before and after, 4096 rays into 20000
-// bodies: 1476, 232; 1000 into 3000: 122, 79; 100 into 50: 48, 47; 1 into 50: 41, 41.
+// bodies: 1476, 223; 1000 into 3000: 122, 78; 100 into 50: 48, 47; 1 into 50: 41, 41.
 constexpr uint32_t RAY_THREADS = 256, RAY_WARPS = RAY_THREADS / 32, RAY_TILE = 64, RAY_CHUNK = 1024;
 template <bool kSpheres, bool kFinish>
 __global__ void __launch_bounds__(RAY_THREADS) k_ray_nearest(DWorld w, RayLaunch R, uint32_t tile, uint32_t chunk) {
@@ -316,7 +330,7 @@ __global__ void __launch_bounds__(RAY_THREADS) k_ray_nearest(DWorld w, RayLaunch
   const uint32_t r0 = blockIdx.y * tile, rays = min(tile, R.n - r0);
   const uint32_t b0 = blockIdx.x * chunk, bodies = min(chunk, R.bodies - b0);
   if (threadIdx.x < rays) {
-    s_ray[threadIdx.x] = R.rays[r0 + threadIdx.x];
+    s_ray[threadIdx.x] = loadRay(R, r0 + threadIdx.x);
     s_best[threadIdx.x] = NO_HIT;
   }
   for (uint32_t b = threadIdx.x; b < bodies; b += RAY_THREADS) {
@@ -378,8 +392,9 @@ __global__ void __launch_bounds__(RAY_THREADS) k_ray_nearest(DWorld w, RayLaunch
 
 __global__ void k_ray_finish(DWorld w, RayLaunch R) {
   const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r < R.n) finishRay(w, R, r, R.rays[r], R.best[r]);
+  if (r < R.n) finishRay(w, R, r, loadRay(R, r), R.best[r]);
 }
+static_assert(sizeof(avbd_ray) == sizeof(DRay) && offsetof(avbd_ray, max_distance) == 12 && offsetof(avbd_ray, direction) == 16, "a ray is eight words");
 static_assert(sizeof(avbd_ray_hit) == 2 * sizeof(float4) && offsetof(avbd_ray_hit, point) == 8 && offsetof(avbd_ray_hit, normal) == 20, "a hit is eight words");
 
 // Device scratch owned by the world (grown on demand, freed with it)
@@ -577,25 +592,25 @@ int avbd_raycast(avbd_world* w, const avbd_ray* rays, uint32_t n, const uint32_t
   if (n > AVBD_RAY_MAX) return qfail(w, AVBD_ERR_INVALID, "avbd_raycast: at most " + std::to_string(AVBD_RAY_MAX) + " rays a call");
   if (n_ignore > AVBD_RAY_MAX_IGNORED) return qfail(w, AVBD_ERR_INVALID, "avbd_raycast: at most " + std::to_string(AVBD_RAY_MAX_IGNORED) + " bodies to ignore");
   if (n == 0) return AVBD_OK;
-  std::vector<DRay> rec(n);
+  uint32_t odd = 0u;  // any infinity or NaN at all; then which ray, the origin and direction first
   for (uint32_t k = 0; k < n; k++) {
+    uint32_t u[8];
+    std::memcpy(u, &rays[k], sizeof(u));
+    for (int a : {0, 1, 2, 4, 5, 6}) odd |= (u[a] & 0x7f800000u) == 0x7f800000u;
+    odd |= (u[3] & 0x7fffffffu) > 0x7f800000u;
+  }
+  for (uint32_t k = 0; odd && k < n; k++) {
     const avbd_ray& r = rays[k];
     for (int a = 0; a < 3; a++)
       if (!std::isfinite(r.origin[a]) || !std::isfinite(r.direction[a])) return qfail(w, AVBD_ERR_INVALID, "ray " + std::to_string(k) + ": non-finite");
     if (std::isnan(r.max_distance)) return qfail(w, AVBD_ERR_INVALID, "ray " + std::to_string(k) + ": NaN distance");
-    // normalised in double (raycast.ts:193-196); a zero direction stays zero
-    double l = std::sqrt(double(r.direction[0]) * r.direction[0] + double(r.direction[1]) * r.direction[1] + double(r.direction[2]) * r.direction[2]);
-    if (!(l > 0.0)) l = 1.0;
-    const float maxd = r.max_distance > 3.0e38f ? 3.0e38f : r.max_distance;
-    rec[k].o = make_float4(r.origin[0], r.origin[1], r.origin[2], maxd);
-    rec[k].d = make_float4(float(r.direction[0] / l), float(r.direction[1] / l), float(r.direction[2] / l), 0.0f);
   }
   cudaSetDevice(w->device);
   cudaError_t e = growBuffer(w, &w->rayBuf, w->rayCap, size_t(n) * sizeof(DRay) / sizeof(float4));
   if (e == cudaSuccess) e = growBuffer(w, &w->rayBest, w->rayBestCap, n);
   if (e == cudaSuccess) e = growBuffer(w, &w->rayHits, w->rayHitsCap, 2 * size_t(n));
   if (e == cudaSuccess) e = growBuffer(w, &w->rayBounds, w->rayBoundsCap, w->n);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(w->rayBuf, rec.data(), n * sizeof(DRay), cudaMemcpyHostToDevice, w->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(w->rayBuf, rays, n * sizeof(avbd_ray), cudaMemcpyHostToDevice, w->stream);
   if (e == cudaSuccess) {
     RayLaunch R{};
     R.rays = reinterpret_cast<const DRay*>(w->rayBuf);
@@ -607,12 +622,12 @@ int avbd_raycast(avbd_world* w, const avbd_ray* rays, uint32_t n, const uint32_t
     R.nIgnore = n_ignore;
     R.mask = mask;
     for (uint32_t k = 0; k < n_ignore; k++) R.ignore[k] = ignore[k];
-    // rays a block: enough blocks for two an SM, a warp a ray at the least; still too few blocks: a quarter
+    // rays a block: enough blocks for two an SM, a warp a ray at the least; still fewer than SMs: a quarter
     // of the bodies each
     uint32_t chunk = RAY_CHUNK, chunks = std::max(1u, grid_for(w->n, chunk));
     const uint32_t tile = std::min(RAY_TILE, std::max(RAY_WARPS, grid_for(uint32_t(uint64_t(n) * chunks / 296u), RAY_WARPS) * RAY_WARPS));
     const uint32_t tiles = grid_for(n, tile);
-    if (chunks > 1u && chunks * tiles < 296u) {
+    if (chunks > 1u && chunks * tiles < 148u) {
       chunk = RAY_CHUNK / 4u;
       chunks = grid_for(w->n, chunk);
     }

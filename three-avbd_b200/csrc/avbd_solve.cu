@@ -1825,11 +1825,10 @@ int solve_grid_blocks(int device) {
 
 // The launch of a world of n bodies: `blocks` of them, or, for 0, by size. Up to SMALL_SOLVE bodies
 // the sweep is a chain of colours, each waiting on the one before with few chunks a warp: one block an
-// SM with all its registers is faster (3001 bodies: solve 0.203 ms against 0.233), and fewer blocks
+// SM with all its registers is faster (5000 bodies: a solve of 227 us against 262), and fewer blocks
 // meet sooner at the barriers between the topology's phases, so long as a colour's rows still get a
-// lane each (a block for 16 bodies; 48 boxes: a step of 82 us against about 150 with every block). Past
-// it the chunks outnumber the warps and two blocks an SM win (20000 bodies: 0.369 ms against 0.398;
-// 100000: 1.30 against 1.60).
+// lane each (48 boxes, a block for 16 bodies: 121; for 32: 134; for 64: 168). Past it the chunks outnumber
+// the warps and two blocks an SM win (12000 bodies: 298 against 336, 16000: 350 against 410).
 constexpr uint32_t SMALL_SOLVE = 8192;
 cudaError_t launch_topology_solve(const DWorld& w, const StepParams& p, int blocks, int maxBlocks, int sms, cudaStream_t s) {
   const bool one = p.n <= SMALL_SOLVE && blocks <= sms;
