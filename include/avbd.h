@@ -261,7 +261,8 @@ int avbd_hull_storage(const avbd_world* world, uint32_t* top, uint32_t* capacity
 int avbd_seed_contacts(avbd_world* world, const avbd_manifold* manifolds, uint32_t n_manifolds, const avbd_contact* contacts,
                        uint32_t n_contacts);
 /* fixedColors (gpu/solver.ts:560, 2130-2134): one colour per body (AVBD_NO_COLOR for none), or
- * NULL to return to the Jones-Plassmann colouring. */
+ * NULL to return to the Jones-Plassmann colouring. Bodies of one colour that touch are solved side by
+ * side, in no given order. */
 int avbd_set_fixed_colors(avbd_world* world, const uint32_t* colors, uint32_t n);
 
 /* step() (gpu/solver.ts:2112-2295): n steps, enqueued on the world's stream (asynchronous). */

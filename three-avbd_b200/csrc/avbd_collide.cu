@@ -46,6 +46,7 @@ __device__ void rotateCounters(const DWorld& w, const StepParams& p) {
   c[C_MANIFOLDS] = 0;
   c[C_OVERFLOW] = 0;
   c[C_CLASHES] = 0;
+  c[C_SAME_COLOR] = 0;
   c[C_COLORS] = 0;
   c[C_ROUNDS] = 0;
   c[C_ERROR] = 0;

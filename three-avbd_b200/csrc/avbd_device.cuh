@@ -43,9 +43,11 @@ enum : int { K_RA = 0, K_RB = 1, K_PEN = 2, K_LAM = 3 };
 enum : int {
   C_PAIRS = 0, C_CONTACTS = 1, C_MANIFOLDS = 2, C_OVERFLOW = 3, C_CLASHES = 4, C_COLORS = 5, C_ROUNDS = 6, C_ERROR = 7,
   C_PREV_PAIRS = 8, C_ADJ = 9, C_INC = 10, C_DYN = 11, C_STEP = 12, C_PENDING = 16,  // 16..16+2*MAX_ROUND_PAIRS: pending counts per round pair
+  C_SAME_COLOR = 96,  // set: a pair or joint joins two bodies of one colour
   COUNTER_WORDS = 128,
 };
 constexpr int MAX_ROUND_PAIRS = 32;
+static_assert(C_PENDING + 2 * MAX_ROUND_PAIRS + 2 <= C_SAME_COLOR && C_SAME_COLOR < COUNTER_WORDS, "counter words");
 constexpr int MAX_CLOCKS = 1023;  // barrier timestamps kept per step
 constexpr int CLOCK_T0 = MAX_CLOCKS + 1, CLOCK_WORDS = MAX_CLOCKS + 2;
 constexpr int STAT_WORDS = 16;    // collision ns, solve ns, then counters (pairs, contacts, manifolds, adjacency, incidences, dynamic, colours, rounds, launches, error)

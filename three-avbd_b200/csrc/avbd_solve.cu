@@ -1032,8 +1032,9 @@ __device__ __forceinline__ void issueRow(const DWorld& w, const StepParams& p, u
 // The tags a lane waits for. A dynamic partner of an earlier colour must have moved in this iteration;
 // one of a later colour, in the one before, and it also updates the shared rows, after the pose. A
 // static partner and the rows this body updates itself are always there. A partner of the same colour
-// (only where the colour cap forced a clash) is not waited for within the iteration: the
-// colour-by-colour sweep runs such pairs side by side too.
+// (colours given by the caller, or more bodies touching one another than there are colours) is waited for
+// up to the iteration before, its pose and its rows: the colour-by-colour sweep runs such pairs side by
+// side too.
 __device__ __forceinline__ uint32_t needPose(uint32_t partnerWord, uint32_t it) {
   return (partnerWord & PARTNER_DYNAMIC) ? ((partnerWord & PARTNER_EARLIER) ? it + 1u : it) : 0u;
 }
@@ -1109,7 +1110,7 @@ __device__ inline bool flowJoint(const DWorld& w, uint2 inc, uint32_t it, Pose& 
 __device__ __forceinline__ bool flowLanes(const DWorld& w, const StepParams& p, const LaneJob& J, uint32_t it) {
   const uint32_t lane = threadIdx.x & 31u;
   const float dt2 = p.dt * p.dt;
-  const bool active = J.active, last = it + 1u == (uint32_t)p.iterations;
+  const bool active = J.active, last = it + 1u == (uint32_t)p.iterations && ldv(&w.counters[C_SAME_COLOR]) == 0u;
   const uint32_t L = J.L, sub = J.sub, body = J.body, e1 = J.e1;
   Pose own;
   Acc acc;
@@ -1176,7 +1177,9 @@ __device__ __forceinline__ bool flowLanes(const DWorld& w, const StepParams& p, 
       dualView(v, own, p, pen, lam, key);
       float4* pt = w.cPt[p.cur] + 4 * size_t((inc.x & ~OWNER_BIT) - p.nj);
       if (key != __float_as_uint(v.ra.w)) pt[K_RA].w = __uint_as_float(key);
-      // the last iteration leaves the record as the contact layout has it, C0's parts in place of the tags
+      // The last iteration leaves the record as the contact layout has it, C0's parts in place of the
+      // tags: the partner, of an earlier colour, has read the row before. A partner of the same colour
+      // may still be waiting for a tag here, which C0's bits are not: then restoreC0 puts C0 back.
       stWord(pt + K_PEN, pen.x, pen.y, pen.z, last ? __float_as_uint(pen.w) : it + 1u);
       stWord(pt + K_LAM, lam.x, lam.y, lam.z, last ? __float_as_uint(lam.w) : it + 1u);
     }
@@ -1217,6 +1220,20 @@ __device__ __noinline__ float3 windAccel(const StepParams& p, float t, float3 x,
   const float un = dot3(u, n);
   const float3 ut = u - n * un;
   return n * (k * un * fabsf(un) / (1.0f + 2.0f * p.dt * k * fabsf(un))) + ut * (0.06f * k * len3(ut));
+}
+
+// C0's tangential parts back into the records of a step whose sweep kept its tags to the end
+__device__ __forceinline__ void restoreC0(const DWorld& w, const StepParams& p, uint32_t pairs, uint32_t tid, uint32_t T) {
+  for (uint32_t m = tid; m < pairs; m += T) {
+    const uint4 ids = w.mIds[p.cur][m];
+    if (!dynBody(w, (int)ids.x) && !dynBody(w, (int)ids.y)) continue;  // not swept: its record was never tagged
+    for (uint32_t k = 0; k < (ids.w & 15u); k++) {
+      const float2 c0 = w.c0t[size_t(ids.z) + k];
+      float4* pt = w.cPt[p.cur] + 4 * (size_t(ids.z) + k);
+      pt[K_PEN].w = c0.x;
+      pt[K_LAM].w = c0.y;
+    }
+  }
 }
 
 // --- the kernel -----------------------------------------------------------------------------------------------
@@ -1478,6 +1495,7 @@ __device__ void topologySolve(const DWorld& w, const StepParams& p, Team& team) 
     if (tid == 0) atomicOr(&ctr[C_ERROR], ERR_INC_OVERFLOW);
     return;  // uniform: every block read the same total after the barrier
   }
+  bool sameColor = false;
   for (uint32_t s = tid; s < numDyn; s += T) {
     uint32_t b = w.colorBodies[s];
     uint32_t colB = w.colorA[b] & 0xffu;
@@ -1491,6 +1509,7 @@ __device__ void topologySolve(const DWorld& w, const StepParams& p, Team& team) 
         uint32_t colO = w.colorA[other] & 0xffu;
         earlier = colO < colB;
         owner = earlier || (colO == colB && other < b);
+        sameColor = sameColor || colO == colB;
       }
       uint32_t flag = owner ? OWNER_BIT : 0u;
       uint32_t partner = ent.w | (earlier ? PARTNER_EARLIER : 0u);
@@ -1499,6 +1518,7 @@ __device__ void topologySolve(const DWorld& w, const StepParams& p, Team& team) 
         for (uint32_t k = 0; k < cnt; k++) w.incList[out++] = make_uint2((nj + (c - nj) * MAX_CONTACTS + k) | flag, partner);
     }
   }
+  if (Team::kDataflow && sameColor) ctr[C_SAME_COLOR] = 1u;
   if constexpr (Team::kDataflow) {
     // the lane table of the dataflow sweep: per colour, its lanes in lane-space order, each with its
     // body, first row, the body's row end and (L, sub)
@@ -1682,6 +1702,7 @@ __device__ void topologySolve(const DWorld& w, const StepParams& p, Team& team) 
       if (!flowLanes(w, p, J, j / mine)) break;
     }
     GSYNC
+    if (p.iterations > 0 && ldv(&ctr[C_SAME_COLOR]) != 0u) restoreC0(w, p, npairs, tid, T);
   } else {
     for (int it = 0; it < p.iterations; it++) {
       for (uint32_t c = 0; c < numColors; c++) {
