@@ -81,3 +81,41 @@ def test_every_block_size_gives_the_same_gradients(cuda_lib, bodies):
         grads.append(g[0])
     for g in grads[1:]:
         assert np.abs(g - grads[0]).max() <= 1e-7 * np.abs(grads[0]).max()
+
+
+@pytest.mark.parametrize('bodies, steps_clashing', [(4, 30), (16, 30), (16, 7), (40, 30), (70, 30)])
+def test_touching_bodies_of_one_color(cuda_lib, bodies, steps_clashing):
+    """A recording whose last `steps_clashing` steps have every body in one colour, touching ones among them:
+    the tape solves such bodies one after another, by index, and so does the replay. Its gradients are the
+    tape's, beside a properly coloured world's in the same batch (to the tolerances of
+    test_gpu_adjoint_matches_the_tape_adjoint)."""
+    from oracle import Adjoint
+    steps = 30
+    A = Oracle(tumbling_world(np.random.default_rng(bodies), bodies)).adjoint(steps)
+    proper, p0 = A.export(), A.nominal()
+    dyn = proper['bodies'].reshape(-1, 13)[:, 11] != 0
+    man = proper['man_bodies'].reshape(-1, 2)[proper['step_man'][steps - steps_clashing]:]
+    assert (dyn[man[:, 0]] & dyn[man[:, 1]]).any()
+    clash = dict(proper)
+    colors, ncol = proper['colors'].reshape(steps, -1).copy(), proper['ncol'].copy()
+    colors[steps - steps_clashing:] = np.where(dyn, 0, -1)
+    ncol[steps - steps_clashing:] = 1
+    clash['colors'], clash['ncol'] = colors.reshape(-1), ncol
+    pt = p0.copy()
+    pt[0::8] += np.random.default_rng(7).normal(0, 0.2, A.n)
+    recs = [clash, proper]
+    tapes = [Adjoint.from_record(r, p0) for r in recs]
+    targets = [t.loss(pt, final=True)[1] for t in tapes]
+    adj = avbd_b200.Adjoint(recs, checkpoint=4)
+    adj.set_target(np.concatenate([t.reshape(-1) for t in targets]))
+    P = np.tile(p0, 2)
+    loss_f, _ = adj.forward(P)
+    loss, g = adj.backward(P)
+    adj.destroy()
+    assert np.allclose(loss, loss_f, rtol=1e-12)
+    for w, (tape, target) in enumerate(zip(tapes, targets)):
+        tape.set_target(target)
+        L, gc = tape.gradient(p0)
+        gw, gc = g.reshape(2, -1, 8)[w][dyn], gc.reshape(-1, 8)[dyn]
+        assert abs(L - loss[w]) < 1e-9 * abs(L), w
+        assert np.abs(gw - gc).max() < 1e-5 * np.abs(gc).max(), w

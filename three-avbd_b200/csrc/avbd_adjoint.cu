@@ -138,7 +138,7 @@ __device__ inline StepView viewOf(const AdjDev& D, int s, int w) {
 }
 
 constexpr int ADJ_MAX_COLORS = 64;
-constexpr int ADJ_GROUP = 32;  // bodies of one colour solved together, a thread each
+constexpr int ADJ_GROUP = 32;  // bodies of one colour solved together, a thread each (s_group)
 constexpr int ADJ_ROW = 27;    // an incidence's share of its body's system: H's lower triangle, g
 constexpr int ADJ_OWN = 15;    // in the reverse sweep: its own body's pose, step-start pose and friction cotangents
 
@@ -149,6 +149,7 @@ __shared__ int s_colStart[ADJ_MAX_COLORS + 1];
 __shared__ int s_colBody[ADJ_MAX_BODIES];
 __shared__ int s_posOf[ADJ_MAX_BODIES];
 __shared__ int s_nSolved;
+__shared__ int s_group;  // ADJ_GROUP, or 1 in a step in which bodies of one colour touch: they are solved one after another
 __shared__ int s_incStart[ADJ_MAX_BODIES + 1];
 __shared__ int s_color[ADJ_MAX_BODIES];
 // Dynamic shared memory: a chunk of incidences, a row each (a block's threads; its share of the body's
@@ -179,6 +180,7 @@ __device__ inline double* floorHb(const AdjDev& D, int i) { return D.floorWork +
 
 __device__ void buildIncidence(const AdjDev& D, const StepView& v) {
   const int tid = threadIdx.x;
+  if (tid == 0) s_group = ADJ_GROUP;
   for (int i = tid; i <= ADJ_MAX_COLORS; i += blockDim.x) s_colStart[i] = 0;
   for (int b = tid; b < v.nb; b += blockDim.x) s_color[b] = v.color[b];
   __syncthreads();
@@ -221,6 +223,7 @@ __device__ void buildIncidence(const AdjDev& D, const StepView& v) {
     const int pa = s_posOf[ab.x], pb = s_posOf[ab.y];
     if (pa >= 0) atomicAdd(&s_incStart[pa + 1], 1);
     if (pb >= 0) atomicAdd(&s_incStart[pb + 1], 1);
+    if (pa >= 0 && pb >= 0 && s_color[ab.x] == s_color[ab.y]) s_group = 1;
   }
   __syncthreads();
   if (tid == 0)
@@ -499,8 +502,8 @@ __device__ void stepForward(const AdjDev& D, int s, int w, int slot) {
   };
   for (int it = 0; it < D.I; it++) {
     for (int c = 0; c < v.ncol; c++) {  // the colour's bodies in groups, a thread each
-      for (int g0 = s_colStart[c]; g0 < s_colStart[c + 1]; g0 += ADJ_GROUP) {
-        const int g1 = min(g0 + ADJ_GROUP, s_colStart[c + 1]);
+      for (int g0 = s_colStart[c]; g0 < s_colStart[c + 1]; g0 += s_group) {
+        const int g1 = min(g0 + s_group, s_colStart[c + 1]);
         groupRows(D, v, wpt, g0, g1, D.lam, D.pen, livePose);
         if (threadIdx.x < g1 - g0) {
           const int gb = v.b0 + s_colBody[g0 + threadIdx.x];
@@ -750,7 +753,8 @@ __device__ inline void incidenceVjp(const AdjDev& D, const StepView& v, int wpt,
     atomicAdd3(&D.gIpos[other], isA ? gXb0 : gXa0);
     atomicAdd4(&D.gIrot[other], isA ? gQb0 : gQa0);
   }
-  // a point has one incidence in a colour: nothing else touches its values here
+  // bodies that touch are never in one group (s_group): a point has one incidence here, and nothing else
+  // touches its values
   D.gLam[wpt + lk] += gLam;
   D.gPen[wpt + lk] += gPen;
   D.gC0[wpt + lk] += gC0;
@@ -766,18 +770,19 @@ __device__ inline void incidenceVjp(const AdjDev& D, const StepView& v, int wpt,
   out[10] = oQ0.x, out[11] = oQ0.y, out[12] = oQ0.z, out[13] = oQ0.w;
 }
 
-// The primal updates of colour c's bodies at positions g0..g1 at iteration it, reversed (poses read
-// from the snapshots the sweep read: partners of earlier colours at iteration it, the rest at
+// The primal updates of the bodies of one colour at positions g0..g1 at iteration it, reversed (poses
+// read from the snapshots the sweep read: partners solved before them at iteration it, the rest at
 // it - 1; the points' values after the dual of iteration it - 1). Thread tid < g1 - g0 owns body
 // position g0 + tid; the incidences are spread over all threads.
-__device__ void primalGroupVjp(const AdjDev& D, const StepView& v, int wpt, int it, int c, int g0, int g1) {
+__device__ void primalGroupVjp(const AdjDev& D, const StepView& v, int wpt, int it, int g0, int g1) {
   const int tid = threadIdx.x, nbg = g1 - g0;
   const double dt2 = D.dt * D.dt;
   const size_t prevSn = (size_t)it * D.nb, curSn = (size_t)(it + 1) * D.nb;
   const D3* lamIn = D.snLam + (size_t)it * D.W * D.maxPts;
   const D3* penIn = D.snPen + (size_t)it * D.W * D.maxPts;
   auto poseOf = [&](int b, D3& x, D4& q) {
-    const size_t o = D.dynamic[b] && v.color[b - v.b0] < c ? curSn : prevSn;
+    const int p = s_posOf[b - v.b0];
+    const size_t o = p >= 0 && p < g0 ? curSn : prevSn;
     x = D.snPos[o + b];
     q = D.snRot[o + b];
   };
@@ -996,8 +1001,8 @@ __device__ void stepBackward(const AdjDev& D0, int s, int w, size_t slot) {
   for (int it = D.I - 1; it >= 0; it--) {
     for (int lk = threadIdx.x; lk < np; lk += blockDim.x) dualVjp(D, v, wpt, it, v.p0 + lk);
     __syncthreads();
-    for (int c = v.ncol - 1; c >= 0; c--)  // the colour's bodies in groups (order within a colour is free)
-      for (int g0 = s_colStart[c]; g0 < s_colStart[c + 1]; g0 += ADJ_GROUP) primalGroupVjp(D, v, wpt, it, c, g0, min(g0 + ADJ_GROUP, s_colStart[c + 1]));
+    for (int c = v.ncol - 1; c >= 0; c--)  // the colour's bodies in groups, the last solved first
+      for (int g1 = s_colStart[c + 1]; g1 > s_colStart[c]; g1 -= s_group) primalGroupVjp(D, v, wpt, it, max(g1 - s_group, s_colStart[c]), g1);
   }
   // points' warm starts and C(x-) (the start poses' cotangents gather in gIpos/gIrot)
   const int prevFirst = s > 0 ? D.ptFirst[(s - 1) * (D.W + 1) + w] : 0;
