@@ -119,3 +119,27 @@ def test_touching_bodies_of_one_color(cuda_lib, bodies, steps_clashing):
         gw, gc = g.reshape(2, -1, 8)[w][dyn], gc.reshape(-1, 8)[dyn]
         assert abs(L - loss[w]) < 1e-9 * abs(L), w
         assert np.abs(gw - gc).max() < 1e-5 * np.abs(gc).max(), w
+
+
+@pytest.mark.parametrize('worlds', [1, 200, 300])
+def test_adjoints_side_by_side(cuda_lib, worlds):
+    """An adjoint of many points still runs, and gives what it gave, after one of few points was made for the
+    same number of worlds, and the other way round."""
+    made = []
+    for bodies in (70, 2, 40):
+        A = Oracle(tumbling_world(np.random.default_rng(bodies), bodies)).adjoint(30)
+        adj = avbd_b200.Adjoint([A.export()] * worlds, checkpoint=4)
+        adj.set_target(np.zeros(7 * A.n * worlds))
+        P = np.tile(A.nominal(), worlds)
+        made.append((adj, P, adj.forward(P), adj.backward(P)))
+    points = [adj.info()['max_points'] for adj, _, _, _ in made]
+    assert points[1] < points[2] < points[0]
+    for adj, P, (loss, fin), (_, g) in made + made[::-1]:
+        again, fin2 = adj.forward(P)
+        loss_b, g2 = adj.backward(P)
+        assert np.array_equal(again, loss) and np.array_equal(fin2, fin) and np.array_equal(loss_b, loss)
+        # atomics of two runs may add in other orders: a double's rounding (1e-16) times the solves' condition
+        # (1e7), a hundred of them in a row
+        assert np.abs(g2 - g).max() <= 1e-7 * np.abs(g).max()
+    for adj, _, _, _ in made:
+        adj.destroy()

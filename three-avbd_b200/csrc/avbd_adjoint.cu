@@ -1188,7 +1188,8 @@ bool aupload(avbd_adjoint* a, const T** dst, const T* src, size_t n) {
 bool adjAllocWork(avbd_adjoint* a) {
   AdjDev& D = a->d;
   a->threads = blockThreads(D.W);
-  const int bytes = int(adjSharedBytes(a->threads, D.maxPts));
+  // a kernel's limit is the process's, not the handle's: the same for every handle, whatever its points
+  const int bytes = int(adjSharedBytes(a->threads, ADJ_MAX_POINTS));
   for (const void* k : {a->forwardKernel(), a->backwardKernel()})
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
   const size_t W = size_t(D.W), K = size_t(D.K), nb = size_t(D.nb);
