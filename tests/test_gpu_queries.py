@@ -220,3 +220,116 @@ def test_pose_capture_frames_match_the_world_and_round_trip(cuda_lib):
     assert len(cap.read()[0]) == 1
     cap.destroy()
     w.destroy()
+
+
+def _turned(rng, length2):
+    """A random rotation scaled to the squared length, as f32."""
+    q = rng.standard_normal(4)
+    return (q / np.linalg.norm(q) * np.sqrt(length2)).astype(np.float32)
+
+
+def _frame(q):
+    """The matrix by which the trace takes a world offset into the body's frame."""
+    return np.stack([queries.rotate(queries.conj(q.astype(float)), np.eye(3)[k]) for k in range(3)], 1)
+
+
+@pytest.mark.parametrize('shape, length2, distance', [
+    ('box', 0.9997, 2.0), ('box', 0.9991, 2.0), ('box', 0.99993, 30.0), ('box', 1.0009, 3.0),
+    ('sphere', 0.9991, 2.0), ('sphere', 1.0009, 60.0), ('sphere', 1.00002, 200.0), ('sphere', 0.999995, 5.0), ('sphere', 1.0000015, 500.0)])
+def test_raycast_grazes_bodies_of_inexact_rotation(cuda_lib, shape, length2, distance):
+    """Rotations a little off unit length, as typed by hand, change what a ray hits: a box is as much larger or
+    smaller as the rotation stretches, and a sphere more the farther the ray comes from. Rays at the edge of
+    what the restatement hits, most of them outside the body's own bounding sphere. What the device finds is
+    compared where the hit or miss holds for the body made smaller and larger: by 1e-4, and a sphere's squared
+    radius also by ten f32 roundings of the squared distance, which its discriminant cancels."""
+    rng = np.random.default_rng(17)
+    size = np.array([1.0, 0.6, 0.8] if shape == 'box' else [1.0, 1.0, 1.0])
+    bound = np.sqrt((size ** 2).sum()) / 2 if shape == 'box' else 0.5
+    hit = outside = missed = 0
+    for _ in range(12):
+        s = Scene('one body')
+        at = rng.uniform(-1, 1, 3)
+        s.box(size, 0, 0.5, at) if shape == 'box' else s.sphere(0.5, 0, 0.5, at)
+        s.bodies[0].rot = [float(x) for x in _turned(rng, length2)]
+        w = avbd_b200.CudaSolver3D(s)
+        body = w.read_bodies()[0]
+        small, large = body.copy(), body.copy()
+        slack = 1.2e-6 * distance ** 2 if shape == 'sphere' else 0.0
+        small['size'] = 2 * np.sqrt(np.maximum(0.0, (size / 2 * (1 - 1e-4)) ** 2 - slack))
+        large['size'] = 2 * np.sqrt((size / 2 * (1 + 1e-4)) ** 2 + slack)
+        stretch = _frame(body['rot'])
+        n = 120
+        o, d = np.zeros((n, 3), np.float32), np.zeros((n, 3), np.float32)
+        for k in range(n):
+            if shape == 'box':  # past a corner, across the direction to it
+                corner = np.linalg.solve(stretch, size / 2 * rng.choice([-1, 1], 3))
+                across = np.cross(corner, rng.standard_normal(3))
+                aim, along = corner * rng.uniform(1 - 3e-3, 1 + 1e-3), across / np.linalg.norm(across)
+            else:  # past the silhouette, which the stretch moves by up to 4 |e| of the squared distance
+                along, x = rng.standard_normal(3), rng.standard_normal(3)
+                along /= np.linalg.norm(along)
+                x -= along * (x @ along)
+                extra = 4 * (length2 - 1) * distance ** 2
+                aim = x / np.linalg.norm(x) * np.sqrt(0.25 * rng.uniform(0.99, 1.01) + extra * rng.uniform(0, 1.1))
+            o[k] = body['pos'].astype(float) + aim - along * distance
+            d[k] = along
+        hits = w.raycast(o, d)
+        w.destroy()
+        for k in range(n):
+            dk = d[k].astype(float)
+            dk = (dk / np.linalg.norm(dk)).astype(np.float32)
+            rel = body['pos'].astype(float) - o[k]
+            perp = np.sqrt(max(0.0, rel @ rel - (rel @ dk) ** 2))
+            inner, outer = (queries.ray_trace(b, None, o[k], dk, 3e38) for b in (small, large))
+            if inner is not None:
+                assert hits['body'][k] == 0, (k, perp)
+                hit += 1
+                outside += perp > bound * (1 + 1e-5)
+            elif outer is None:
+                assert hits['body'][k] == -1, (k, perp)
+                missed += 1
+    assert hit >= 100 and missed >= 100
+    assert outside >= (20 if shape == 'box' and length2 < 0.9998 or shape == 'sphere' and length2 > 1 else 0)
+
+
+@pytest.mark.parametrize('n, rays', [(31, 65), (400, 900), (1023, 400), (2500, 500), (1100, 4800)])
+def test_raycast_passes_over_no_hit(cuda_lib, n, rays):
+    """Near and far rays into a pile of long, flat, round and unnormalised bodies, against the restatement: a
+    miss on the device must be one of the bodies made smaller by the tolerance, a hit one of the bodies made
+    larger, and the body that the device names must lie as near as the nearest one."""
+    rng = np.random.default_rng(n + rays)
+    scene = drop_pile(n, seed=4, spacing=1.3, layers=3)
+    for b in scene.bodies[1::3]:
+        b.size = [float(x) for x in rng.uniform(0.05, 1.5, 3)] if b.shape == 0 else b.size
+    for b in scene.bodies[1::4]:
+        b.rot = [float(x * rng.choice([0.99985, 1.0001, 0.9, 1.3])) for x in b.rot]
+    w = avbd_b200.CudaSolver3D(scene)
+    bodies = w.read_bodies()
+    at = bodies['pos'][rng.integers(1, n + 1, rays)] + rng.normal(0, 0.3, (rays, 3))
+    d = rng.standard_normal((rays, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    o = (at - d * rng.choice([0.5, 3.0, 100.0], (rays, 1))).astype(np.float32)
+    hits = w.raycast(o, d)
+    filters = np.full((n + 1, 2), 0xFFFFFFFF, np.uint32)
+    agree = 0
+    for k in range(0, rays, max(1, rays // 24)):
+        dk = d[k].astype(np.float32).astype(float)
+        dk = (dk / np.linalg.norm(dk)).astype(np.float32)
+        # f32 rounds a ray's offset to 2^-23 of its distance, a few times over; a grazing ray moves along by
+        # the root of that
+        tol = 2e-6 * (1.0 + float(np.linalg.norm(o[k] - at[k])))
+        small, large = bodies.copy(), bodies.copy()
+        small['size'] = np.maximum(0.0, small['size'] - np.float32(20 * tol))
+        large['size'] += np.float32(20 * tol)
+        inner, outer = queries.raycast(small, None, filters, o[k], dk), queries.raycast(large, None, filters, o[k], dk)
+        b, t = int(hits['body'][k]), float(hits['distance'][k])
+        if b < 0:
+            assert inner is None, f'ray {k}: missed body {inner[0]}'
+            continue
+        assert outer is not None and t >= outer[1] - 20 * tol, f'ray {k}: body {b} at {t}, the nearest is {outer}'
+        assert inner is None or t <= inner[1] + 20 * tol, f'ray {k}: body {b} at {t}, past body {inner[0]} at {inner[1]}'
+        own = queries.ray_trace(large[b], None, o[k], dk, 3e38)
+        assert own is not None and t >= own[0] - 20 * tol
+        agree += 1
+    assert agree >= 8
+    w.destroy()

@@ -257,16 +257,19 @@ __device__ float rayTrace(const DWorld& w, uint32_t b, const DRay& r, float3& n)
 }
 
 // A sphere that holds every point of body i that rayTrace can hit, xyz and squared radius: -inf for a
-// body the query skips, +inf (always traced) for a hull, whose planes are not bounded by a record field,
-// and for a rotation that is not of unit length, which would stretch the body.
+// body the query skips, +inf (always traced) for a hull, whose planes are not bounded by a record field.
+// With a rotation whose squared length is off by e, qrotate stretches or shrinks what is across its axis
+// by up to 1 + 4 e, squared. A box grows by that, at most (past 1e-3: +inf). A sphere's trace also takes
+// the ray's turned direction for a unit vector, which brings the ray up to 4 e of its squared distance
+// nearer: within 2e-6, where the solver's own rotations are, nearSphere's margin covers it; past that: +inf.
 __device__ __forceinline__ float4 raySphere(const DWorld& w, const RayLaunch& R, uint32_t i) {
   const float4 pos = w.pos[i], size = w.size[i], q = w.rot[i];
   const float shape = w.avel[i].w;
   const float inf = __int_as_float(0x7f800000);
-  float r2 = (size.x * size.x + size.y * size.y + size.z * size.z) * 0.25f;
-  if (fabsf(shape - 1.0f) < 0.5f) r2 = size.x * size.x * 0.25f;
-  else if (shape > 2.5f) r2 = inf;
-  if (!(fabsf(q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w - 1.0f) < 1e-3f)) r2 = inf;
+  const float e = fabsf(q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w - 1.0f);
+  const bool sphere = fabsf(shape - 1.0f) < 0.5f;
+  float r2 = sphere ? size.x * size.x * 0.25f : (size.x * size.x + size.y * size.y + size.z * size.z) * 0.25f * (1.0f + 5.0f * e);
+  if (shape > 2.5f || !(e < (sphere ? 2.0e-6f : 1.0e-3f))) r2 = inf;
   if (rayIgnores(w, R, i)) r2 = -inf;
   return make_float4(pos.x, pos.y, pos.z, r2);
 }
@@ -278,7 +281,7 @@ __device__ __forceinline__ bool nearSphere(float4 x, float3 o, float3 d) {
   const float along = dot3(rel, d), far2 = dot3(rel, rel);
   float ahead;
   asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(ahead) : "f"(along));
-  return !(far2 - ahead * ahead > x.w + 8.0e-6f * far2);
+  return !(far2 - ahead * ahead > x.w + 1.6e-5f * far2);
 }
 // Every body's sphere, once for all the blocks that read it; resets the keys too
 __global__ void k_ray_prepare(DWorld w, RayLaunch R) {
@@ -307,10 +310,11 @@ __device__ __forceinline__ void finishRay(const DWorld& w, const RayLaunch& R, u
 
 // A tile of rays (blockIdx.y) against a chunk of bodies, whose spheres are staged in shared memory: a warp
 // takes a ray and its lanes the spheres. A ray is traced against a body only where it passes the body's
-// sphere, grown by 8e-6 of the squared distance from the origin (over sixty f32 roundings of it: the
-// test's own, which come to thirteen, and rayTrace's, its sphere discriminant's above all) so that no hit
-// that rayTrace would report is passed over; the pairs that pass are queued and traced a lane each. Tracing every ray against every
-// body read 64 bytes and ran six plane divisions for each pair, and one pair in a thousand hits; tracing
+// sphere, grown by 1.6e-5 of the squared distance from the origin (a sphere's rotation's 4 x 2.3e-6, its
+// own rounding counted, and over fifty f32 roundings: the test's own, which come to thirteen, and
+// rayTrace's, its sphere discriminant's above all) so that no hit that rayTrace would report is passed
+// over; the pairs that pass are queued and traced a lane each. Tracing every ray against every body read
+// 64 bytes and ran six plane divisions for each pair, and one pair in a thousand hits; tracing
 // where the sphere test passed, a lane or two at a time, left few rays waiting on one trace after another.
 // The sphere test is bound by instruction issue. The least (distance bits, body) key is the nearest hit
 // and, among hits at the same distance, the lowest body index, as the reference's two atomic passes find
