@@ -58,3 +58,36 @@ def test_a_world_without_bodies_steps(cuda_lib):
     c = w.read_counters()
     assert c['steps'] == 3 and c['pairs'] == 0 and c['error'] == 0
     w.destroy()
+
+
+@pytest.mark.parametrize('bodies', [3, 48, 700])
+def test_capacity_above_the_population_changes_nothing(cuda_lib, bodies):
+    """Tables made for many more bodies than there are are emptied by other launches than those of a world
+    that is full (the warm-start table past 256 words a thread by a memset): the same steps bit for bit, also
+    with kept manifolds between, and after bodies came that put the world on the other side of the rule."""
+    scene = drop_pile(bodies, seed=3, spacing=1.3, layers=3)
+    records, _, _, _ = avbd_b200.scene_records(scene)
+    more = records[1:].copy()
+    more['pos'][:, 2] += 8.0
+    for f in ('initial_pos', 'inertial_pos'):
+        more[f] = more['pos']
+    out = []
+    for capacity in (2 * bodies + 1, 20000, 300000):
+        w = avbd_b200.CudaSolver3D(body_capacity=capacity)
+        w.params = scene.params
+        w.add_bodies(records)
+        state = []
+        for k in range(12):
+            w.step(2)
+            w.step(1, reuse_manifolds=True)
+            if k == 5:
+                w.add_bodies(more)
+            c = w.read_counters()
+            assert c['error'] == 0 and c['overflow'] == 0
+            state.append((c['pairs'], c['contacts'], w.read_bodies().tobytes()))
+        out.append(state)
+        w.destroy()
+    assert out[0][-1][1] > 0
+    for state in out[1:]:
+        for k, (a, b) in enumerate(zip(out[0], state)):
+            assert a == b, f'round {k}'

@@ -1844,8 +1844,9 @@ void launch_step_stats(const DWorld& w, uint32_t launches, cudaStream_t s) { k_s
 // Host: the collision phase, enqueued on `s`. Returns the number of kernels it launched.
 uint32_t launch_collision(const DWorld& w, const StepParams& p, uint32_t tableSize, bool reuseManifolds, cudaStream_t s) {
   const uint32_t n = p.n;
-  // grid-stride kernels over device-side counts: no more blocks than a small world has work for
-  const uint32_t gs = std::min<uint32_t>(GS_BLOCKS, 1u + n / 16u);
+  // grid-stride kernels over device-side counts, which also clear the cell table: no more blocks than a
+  // small world, and a table made for many more bodies, have work for
+  const uint32_t gs = std::min<uint32_t>(GS_BLOCKS, 1u + std::max(n / 16u, tableSize / 2048u));
   if (reuseManifolds) {
     k_begin<<<1, 1, 0, s>>>(w, p);
     uint32_t launches = 2;

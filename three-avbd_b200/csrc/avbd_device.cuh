@@ -76,6 +76,7 @@ struct StepParams {
   uint32_t fixedColors;  // colours come from the host (validation), no Jones-Plassmann
   uint32_t colorCap;
   uint32_t laneBudget;   // threads the grid's lane classes are sized by (0: the launch's own)
+  uint32_t clearHash;    // the solve empties the warm-start table (else its launch does, by a memset)
   uint32_t rowsPerLane;  // the least rows a lane of a body's group takes (0, 1: as the colour's size asks)
   int cur;               // which manifold/contact buffers this step writes
 };

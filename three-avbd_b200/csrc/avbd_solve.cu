@@ -1250,7 +1250,7 @@ __device__ void topologySolve(const DWorld& w, const StepParams& p, Team& team) 
   const uint32_t ncons = nj + npairs;
 
   // the warm-start table, past its last reader, emptied for the next step (a power of two words)
-  if constexpr (Team::kDataflow) {
+  if (Team::kDataflow && p.clearHash) {
     uint4* h4 = reinterpret_cast<uint4*>(w.hash);
     for (uint32_t i = tid; i < (p.hashMask + 1u) / 4u; i += T) h4[i] = make_uint4(0u, 0u, 0u, 0u);
     if (p.hashMask < 3u && tid <= p.hashMask) w.hash[tid] = 0u;
@@ -1851,6 +1851,7 @@ int solve_grid_blocks(int device) {
 // lane each (48 boxes, a block for 16 bodies: 121; for 32: 134; for 64: 168). Past it the chunks outnumber
 // the warps and two blocks an SM win (12000 bodies: 298 against 336, 16000: 350 against 410).
 constexpr uint32_t SMALL_SOLVE = 8192;
+constexpr uint32_t CLEAR_WORDS = 256;
 cudaError_t launch_topology_solve(const DWorld& w, const StepParams& p, int blocks, int maxBlocks, int sms, cudaStream_t s) {
   const bool one = p.n <= SMALL_SOLVE && blocks <= sms;
   StepParams pc = p;
@@ -1859,8 +1860,16 @@ cudaError_t launch_topology_solve(const DWorld& w, const StepParams& p, int bloc
   if (blocks <= 0) blocks = one ? std::min<int>(sms, std::max<int>(1, int(p.n + 15u) / 16)) : maxBlocks;
   DWorld wc = w;
   void* args[] = {&wc, &pc};
+  // The warm-start table is as long as the pair storage, which may be made for many more bodies than there
+  // are: past CLEAR_WORDS a thread a memset is faster (48 bodies in a world made for a million, a step and
+  // the wait for it: 542 us by the kernel, 213 with the memset and the cell table cleared by blocks enough;
+  // for 100000: 233, 195; for 10000, the last that the kernel clears: 187).
+  const size_t hashWords = size_t(p.hashMask) + 1;
+  pc.clearHash = hashWords <= size_t(blocks) * SOLVE_THREADS * CLEAR_WORDS ? 1u : 0u;
   const void* kernel = one ? (const void*)k_topology_solve<1> : (const void*)k_topology_solve<2>;
-  return cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(SOLVE_THREADS), args, 0, s);
+  const cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(SOLVE_THREADS), args, 0, s);
+  if (e != cudaSuccess || pc.clearHash) return e;
+  return cudaMemsetAsync(w.hash, 0, hashWords * sizeof(uint32_t), s);
 }
 
 }  // namespace avbd
