@@ -91,3 +91,25 @@ def test_capacity_above_the_population_changes_nothing(cuda_lib, bodies):
     for state in out[1:]:
         for k, (a, b) in enumerate(zip(out[0], state)):
             assert a == b, f'round {k}'
+
+
+@pytest.mark.parametrize('n, slabs', [(300, 0), (300, 1), (300, 2), (300, 16), (300, 17), (3000, 60), (33000, 6), (33000, 60)])
+def test_many_large_bodies(cuda_lib, n, slabs):
+    """Large bodies up to the most there may be (64), fixed and moving, through a pile: the walk's places for
+    the first ones and its lanes' strides over the rest, sixteen lanes a body and four, find the restated
+    grid's pairs."""
+    scene = drop_pile(n, seed=n, spacing=1.25, layers=6)
+    rng = np.random.default_rng(n)
+    side = max(abs(x) for b in scene.bodies[1:] for x in b.pos[:2])
+    for k in range(slabs):
+        scene.box([9.0, 9.0, 0.5], 1.0 if k % 3 else 0, 0.5, [*rng.uniform(-side, side, 2), float(rng.uniform(0, 8))])
+    w = avbd_b200.CudaSolver3D(scene)
+    before = w.read_bodies()
+    want = _pairs(avbd_b200.find_pairs_noalloc(before)) if n <= 4000 else _pairs(Oracle(scene, fp32=True).pairs())
+    w.step()
+    got = w.read_pairs()
+    assert len(got) == len(_pairs(got)) and _pairs(got) == want
+    first = n + 1
+    assert sum(max(p) >= first for p in want) >= 5 * slabs
+    assert w.read_counters()['error'] == 0
+    w.destroy()

@@ -495,7 +495,7 @@ __device__ inline void largeAgainstLarge(const DWorld& w, const StepParams& p, c
 }
 
 // kLanes lanes a body walk its cells side by side with the cheap tests (cell, sphere, AABB), and the
-// large bodies after them; the candidates that pass go to a per-warp queue in shared memory, and
+// large bodies after them (sphere); the candidates that pass go to a per-warp queue in shared memory, and
 // whenever it holds a warp's worth, the warp takes the full test (the prober's view, the face
 // separation, the no-collide list) one candidate a lane, so that the long test runs on full warps
 // instead of on the few lanes whose walk found one. The walk is bound by its dependent loads (bucket,
@@ -518,7 +518,10 @@ __device__ __forceinline__ void drainQueue(const DWorld& w, const StepParams& p,
   count -= take;
   if (lane < take) testCandidate(w, p, e);
 }
-constexpr uint32_t WALK_LARGE = 14;  // the place after the cells: the large bodies
+// The places after the cells: the first large bodies, one each. Past those the lanes stride the list. (One
+// lane for all of them, and the full test for each: 50 more walls around 20000 bodies were 41 us of
+// collision, around 100000 75; now 4 and 12.)
+constexpr uint32_t WALK_LARGE = 14, WALK_PLACES = 16;
 template <uint32_t kLanes>
 __global__ void __launch_bounds__(PAIR_WALK_THREADS) k_find_pairs(DWorld w, StepParams p) {
   __shared__ uint2 s_queue[PAIR_WALK_THREADS / 32][PAIR_QUEUE];
@@ -529,17 +532,38 @@ __global__ void __launch_bounds__(PAIR_WALK_THREADS) k_find_pairs(DWorld w, Step
   const bool on = i < p.n && enabled(w, i);
   const bool dyn = on && w.size[i].w > 0.0f;
   const bool small = on && w.moment[i].w <= p.largeThreshold;
+  const bool large = small ? dyn || p.anyDynamicLarge : dyn;  // this body is tested against the large ones
   float3 pos = make_float3(0.0f, 0.0f, 0.0f), aabb = pos;
   float radius = 0.0f;
   int4 own = make_int4(0, 0, 0, 0);
-  if (small) {
+  if (on) {
     pos = f3(w.pos[i]);
     radius = w.moment[i].w;
+  }
+  if (small) {
     aabb = aabbOf(w, i);
     own = w.cell[i];
   }
+  auto enqueue = [&](bool push, uint32_t j) {
+    const uint32_t m = __ballot_sync(0xffffffffu, push);
+    if (m) {
+      if (push) Q[count + __popc(m & ((1u << lane) - 1u))] = make_uint2(i, j);
+      count += __popc(m);
+      __syncwarp();
+      if (count >= 32u) drainQueue(w, p, Q, count, lane);
+    }
+  };
+  // a small body against the k-th large one, or a large dynamic body against it (each pair of large bodies
+  // once)
+  auto largeCandidate = [&](uint32_t k, uint32_t& j) -> bool {
+    j = w.large[k];
+    if (small ? !dyn && !(enabled(w, j) && w.size[j].w > 0.0f) : j == i || (j < i && w.size[j].w > 0.0f)) return false;
+    const float3 d = pos - f3(w.pos[j]);
+    const float r = radius + w.moment[j].w;
+    return !(dot3(d, d) > r * r);  // the sphere test, the same in both views
+  };
 #pragma unroll 1
-  for (uint32_t o = lane % kLanes; o - lane % kLanes <= WALK_LARGE; o += kLanes) {
+  for (uint32_t o = lane % kLanes; o - lane % kLanes < WALK_PLACES; o += kLanes) {
     int4 cc = make_int4(0, 0, 0, 0);
     uint32_t k = 0, end = 0;
     if (small && o < WALK_LARGE) {
@@ -549,17 +573,12 @@ __global__ void __launch_bounds__(PAIR_WALK_THREADS) k_find_pairs(DWorld w, Step
       const uint32_t h = cellHash(cc, p.tableMask);
       k = w.cellStart[h];
       end = w.cellEnd[h];
-    } else if (o == WALK_LARGE && ((small && (dyn || p.anyDynamicLarge)) || (!small && dyn))) {
-      end = p.nLarge;
+    } else if (o >= WALK_LARGE && large) {
+      k = o - WALK_LARGE;
+      end = min(k + 1u, p.nLarge);
     }
     auto candidate = [&](uint32_t kk, uint32_t& jj) -> bool {
-      if (o == WALK_LARGE) {
-        // a small body against the large list, or a large dynamic body against it (each pair of large
-        // bodies once)
-        jj = w.large[kk];
-        if (!small) return jj != i && !(jj < i && w.size[jj].w > 0.0f);
-        return dyn || (enabled(w, jj) && w.size[jj].w > 0.0f);
-      }
+      if (o >= WALK_LARGE) return largeCandidate(kk, jj);
       const int4 cj = w.sortedCell[kk];
       jj = (uint32_t)cj.w & 0x7fffffffu;
       const bool dj = ((uint32_t)cj.w & 0x80000000u) != 0u;
@@ -575,14 +594,15 @@ __global__ void __launch_bounds__(PAIR_WALK_THREADS) k_find_pairs(DWorld w, Step
       uint32_t j = 0;
       const bool push = k < end && candidate(k, j);
       k++;
-      const uint32_t m = __ballot_sync(0xffffffffu, push);
-      if (m) {
-        if (push) Q[count + __popc(m & ((1u << lane) - 1u))] = make_uint2(i, j);
-        count += __popc(m);
-        __syncwarp();
-        if (count >= 32u) drainQueue(w, p, Q, count, lane);
-      }
+      enqueue(push, j);
     }
+  }
+#pragma unroll 1
+  for (uint32_t k0 = WALK_PLACES - WALK_LARGE; k0 < p.nLarge; k0 += kLanes) {
+    const uint32_t k = k0 + lane % kLanes;
+    uint32_t j = 0;
+    const bool push = large && k < p.nLarge && largeCandidate(k, j);
+    enqueue(push, j);
   }
   while (count > 0u) drainQueue(w, p, Q, count, lane);
 }
