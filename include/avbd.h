@@ -537,7 +537,7 @@ typedef struct avbd_batch_status {
   uint32_t relayouts; /* times pair storage was laid out again for a world that outgrew it */
   uint32_t collide_threads, collide_blocks, solve_blocks, graphs;
   uint32_t rows_per_lane; /* the solve's least rows a lane of a body's group */
-  uint32_t world_threads; /* the solve's threads a world: 256 (a block a world), 128, 64 or 32 */
+  uint32_t world_threads; /* the solve's threads a world: 256 (a block a world; 512 where collide_threads is), 128, 64 or 32 */
 } avbd_batch_status;
 
 /* The autotuner's measurements: per candidate launch shape (collision block size, solve blocks,
@@ -580,12 +580,15 @@ int avbd_batch_write_all_bodies_async(avbd_batch* batch, const avbd_body* src, u
 int avbd_batch_use_graphs(avbd_batch* batch, int enable);
 int avbd_batch_stream(avbd_batch* batch, void** stream);
 /* Times each candidate launch shape over `steps` real steps and keeps the fastest: the collision
- * block size first, then the solve's threads a world x solve blocks, then four rows a lane. */
+ * block size first, then the solve's threads a world x solve blocks, with no more worlds than SMs the
+ * shape of 512 threads, then four rows a lane. */
 int avbd_batch_tune(avbd_batch* batch, int steps, avbd_batch_tuning* out);
 /* Sets the launch shape the tuner would choose: collision block size (64, 128 or 256), solve blocks
  * (0: as many as fit), the least rows a lane (1 to 8) and the solve's threads a world (256: a block a
- * world; 128, 64 or 32: two, four or eight worlds a block). Every shape gives the same results bit for
- * bit. No counterpart in the reference (it has no batched worlds). */
+ * world; 128, 64 or 32: two, four or eight worlds a block). Collision blocks of 512, with 256 threads a
+ * world, give the solve's blocks 512 threads as well: the shape of a batch of no more worlds than SMs
+ * before either call; one of more worlds has (128, 0, 1, 256). Every shape gives the same results bit
+ * for bit. No counterpart in the reference (it has no batched worlds). */
 int avbd_batch_set_launch(avbd_batch* batch, uint32_t collide_threads, uint32_t solve_blocks, uint32_t rows_per_lane, uint32_t world_threads);
 int avbd_batch_info(avbd_batch* batch, avbd_batch_status* out);
 

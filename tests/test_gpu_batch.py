@@ -265,3 +265,44 @@ def test_few_worlds_and_many_step_alike(cuda_lib, n):
         assert a == c and a['error'] == 0 and a['overflow'] == 0
     few.destroy()
     many.destroy()
+
+
+def test_explicit_launch_shapes_are_the_ones_that_run(cuda_lib):
+    """A batch of no more worlds than SMs takes blocks of 512 threads by itself; a shape that is set, or tuned,
+    is the one reported and kept, also over worlds added later, and all give the same bits. What the tuner
+    chooses can be set on another batch."""
+    scenes = _mixed_scenes()
+    out = []
+    for shape in (None, (64, 0, 1, 256), (128, 0, 1, 256), (256, 12, 1, 256), (512, 0, 1, 256), (512, 5, 1, 256), (128, 0, 1, 64)):
+        n, nj = sum(len(s.bodies) for s in scenes), sum(sum(1 for f in s.forces if f.kind != 'ignore') for s in scenes)
+        b = BatchSolver3D(len(scenes), n, nj, params=scenes[0].params)
+        if shape:
+            b.set_launch(*shape)
+        for s in scenes:
+            b.add_scene(s)
+        b.step(20)
+        b.synchronize()
+        info = b.info()
+        assert info['collide_threads'] == (shape[0] if shape else 512) and info['world_threads'] == (shape[3] if shape else 256)
+        if shape and shape[1]:
+            assert info['solve_blocks'] == shape[1]
+        out.append(np.concatenate([b.read_bodies(i) for i in range(len(scenes))]).tobytes())
+        b.destroy()
+    assert all(o == out[0] for o in out[1:])
+    few, many = _batch_for(scenes), _batch_for([scenes[0]] * 200)
+    for bad in ((512, 0, 1, 128), (512, 10 ** 6, 1, 256), (1024, 0, 1, 256)):
+        with pytest.raises(avbd_b200.AvbdError):
+            few.set_launch(*bad)
+    many.step(1)
+    many.synchronize()
+    assert many.info()['collide_threads'] == 128
+    for b, wide in ((few, True), (many, False)):
+        t = b.tune(2)
+        tried = {(c['collide_threads'], c['world_threads']) for c in t['candidates']}
+        assert {(64, 256), (128, 256), (256, 256)} <= tried and ((512, 256) in tried) == wide
+        other = _batch_for(scenes[:1])
+        other.set_launch(t['collide_threads'], t['solve_blocks'], t['rows_per_lane'], t['world_threads'])
+        assert {k: other.info()[k] for k in ('collide_threads', 'solve_blocks', 'rows_per_lane', 'world_threads')} == {
+            k: b.info()[k] for k in ('collide_threads', 'solve_blocks', 'rows_per_lane', 'world_threads')}
+        other.destroy()
+        b.destroy()

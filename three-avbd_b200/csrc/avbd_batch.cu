@@ -45,6 +45,7 @@ struct avbd_batch {
   uint32_t stepCount = 0;
   // launch shape (the autotuner's choice)
   int sms = 0, collideThreads = 128, collideBlocks = 0, solveBlocks = 0;
+  bool shapeSet = false;     // by the tuner or avbd_batch_set_launch; else launchShape goes by the worlds
   uint32_t rowsPerLane = 1;  // the solve's least rows a lane (bodies per warp), chosen by the tuner
   int worldThreads = 256;    // the solve's threads a world: 256 (a block) or 32 (a warp), chosen by the tuner
   // status of the last step, copied back asynchronously
@@ -247,11 +248,18 @@ int adaptBatch(avbd_batch* b, bool wait) {
   return layoutPairs(b, old);
 }
 
+// Blocks of BATCH_WIDE_THREADS in the collision stand for the wide shape: the solve's block a world has as many
+int solveThreads(const avbd_batch* b) { return b->collideThreads == BATCH_WIDE_THREADS ? BATCH_WIDE_THREADS : b->worldThreads; }
+
 void launchShape(avbd_batch* b) {
   const int nw = int(std::max<size_t>(b->worlds.size(), 1));
+  // No more worlds than SMs, a block each: the step lasts as long as its largest world, and the SM's other
+  // half would stand empty, so a world gets 512 threads. (96 worlds of 16 to 250 bodies, one step and the
+  // readback: 494 us, now 387.)
+  if (!b->shapeSet) b->collideThreads = nw <= b->sms ? BATCH_WIDE_THREADS : 128;
   int cper = std::max(1, batch_collide_blocks_per_sm(b->collideThreads));
   b->collideBlocks = std::min(nw, b->sms * cper);
-  if (b->solveBlocks <= 0) b->solveBlocks = b->sms * std::max(1, batch_solve_blocks_per_sm(b->worldThreads));
+  if (!b->shapeSet || b->solveBlocks <= 0) b->solveBlocks = b->sms * std::max(1, batch_solve_blocks_per_sm(solveThreads(b)));
 }
 
 BatchLaunch makeLaunch(avbd_batch* b) {
@@ -287,14 +295,10 @@ BatchLaunch makeLaunch(avbd_batch* b) {
 cudaError_t enqueueStep(avbd_batch* b, const BatchLaunch& L) {
   cudaMemsetAsync(b->dQueue, 0, 2 * sizeof(uint32_t), b->stream);
   cudaMemsetAsync(b->dStatus, 0, 2 * sizeof(uint32_t), b->stream);
-  // No more worlds than SMs, a block each: the step lasts as long as its largest world, and the SM's other
-  // half would stand empty, so a world gets 512 threads. (96 worlds of 16 to 250 bodies, one step and the
-  // readback: 494 us, now 387.)
-  const bool wide = int(L.nWorlds) <= b->sms && b->solveBlocks >= int(L.nWorlds) && b->worldThreads == BATCH_SOLVE_THREADS;
-  cudaError_t e = launch_batch_collision(L, b->collideBlocks, wide ? 512 : b->collideThreads, b->stream);
+  cudaError_t e = launch_batch_collision(L, b->collideBlocks, b->collideThreads, b->stream);
   if (e != cudaSuccess) return e;
   const int worldsPerBlock = BATCH_SOLVE_THREADS / std::max(32, std::min(b->worldThreads, BATCH_SOLVE_THREADS));
-  e = launch_batch_solve(L, std::min<int>(b->solveBlocks, (int(L.nWorlds) + worldsPerBlock - 1) / worldsPerBlock), wide ? 512 : b->worldThreads, b->stream);
+  e = launch_batch_solve(L, std::min<int>(b->solveBlocks, (int(L.nWorlds) + worldsPerBlock - 1) / worldsPerBlock), solveThreads(b), b->stream);
   if (e != cudaSuccess) return e;
   return cudaMemcpyAsync(b->hStatus, b->dStatus, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, b->stream);
 }
@@ -824,8 +828,9 @@ int avbd_batch_tune(avbd_batch* b, int steps, avbd_batch_tuning* out) {
   float best = INFINITY;
   int bestT = b->collideThreads, bestS = b->solveBlocks, bestW = b->worldThreads;
   uint32_t bestR = b->rowsPerLane;
-  const bool graphs = b->useGraphs;
+  const bool graphs = b->useGraphs, shapeWasSet = b->shapeSet;
   b->useGraphs = false;
+  b->shapeSet = true;
   uint32_t k = 0;
   // one candidate: its mean step time over `steps` after one step that settles storage for the shape
   auto trial = [&](int ct, int sb, uint32_t rpl, int wt) -> int {
@@ -872,6 +877,9 @@ int avbd_batch_tune(avbd_batch* b, int steps, avbd_batch_tuning* out) {
     const int per = std::max(1, batch_solve_blocks_per_sm(worldThreads[wi]));
     for (int sp = 1; sp <= per && !r; sp++) r = trial(collideBest, b->sms * sp, 1, worldThreads[wi]);
   }
+  // few worlds: a block of twice the threads each
+  if (!r && int(b->worlds.size()) <= b->sms)
+    r = trial(BATCH_WIDE_THREADS, b->sms * std::max(1, batch_solve_blocks_per_sm(BATCH_WIDE_THREADS)), 1, BATCH_SOLVE_THREADS);
   // then bodies per warp: four rows a lane at least, in the fastest scope and block count so far
   if (!r) r = trial(bestT, bestS, 4, bestW);
   cudaEventDestroy(e0);
@@ -881,6 +889,7 @@ int avbd_batch_tune(avbd_batch* b, int steps, avbd_batch_tuning* out) {
   b->solveBlocks = bestS;
   b->rowsPerLane = bestR;
   b->worldThreads = bestW;
+  if (r) b->shapeSet = shapeWasSet;
   launchShape(b);
   b->configGen++;
   if (r) return r;
@@ -961,13 +970,14 @@ int avbd_batch_record_status(avbd_batch* b, uint32_t* steps, uint64_t* manifolds
 
 int avbd_batch_set_launch(avbd_batch* b, uint32_t collideThreads, uint32_t solveBlocks, uint32_t rowsPerLane, uint32_t worldThreads) {
   if (!b) return AVBD_ERR_INVALID;
-  if (collideThreads != 64 && collideThreads != 128 && collideThreads != 256)
-    return bfail(b, AVBD_ERR_INVALID, "collision block size must be 64, 128 or 256");
+  const bool wide = collideThreads == uint32_t(BATCH_WIDE_THREADS) && worldThreads == uint32_t(BATCH_SOLVE_THREADS);
+  if (collideThreads != 64 && collideThreads != 128 && collideThreads != 256 && !wide)
+    return bfail(b, AVBD_ERR_INVALID, "collision block size must be 64, 128 or 256 (512 with a block a world)");
   if (rowsPerLane < 1 || rowsPerLane > 8) return bfail(b, AVBD_ERR_INVALID, "rows per lane must be 1 to 8");
   if (worldThreads != 32 && worldThreads != 64 && worldThreads != 128 && worldThreads != 256)
     return bfail(b, AVBD_ERR_INVALID, "threads a world must be 32, 64, 128 or 256");
   cudaSetDevice(b->device);
-  const int per = std::max(1, batch_solve_blocks_per_sm(int(worldThreads)));
+  const int per = std::max(1, batch_solve_blocks_per_sm(wide ? BATCH_WIDE_THREADS : int(worldThreads)));
   if (solveBlocks > uint32_t(b->sms * per))
     return bfail(b, AVBD_ERR_INVALID, "solve blocks beyond " + std::to_string(b->sms * per) + " (the blocks that fit)");
   int r = avbd_batch_synchronize(b);
@@ -976,6 +986,7 @@ int avbd_batch_set_launch(avbd_batch* b, uint32_t collideThreads, uint32_t solve
   b->solveBlocks = int(solveBlocks);  // 0: as many as fit (launchShape)
   b->rowsPerLane = rowsPerLane;
   b->worldThreads = int(worldThreads);
+  b->shapeSet = true;
   launchShape(b);
   b->configGen++;
   return AVBD_OK;

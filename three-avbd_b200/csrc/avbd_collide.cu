@@ -1713,11 +1713,11 @@ __global__ void __launch_bounds__(128) k_narrowphase(DWorld w, StepParams p) {
 // the one or two lanes of a warp that came to it (96 worlds a step 597 us, now 494; 4096 worlds, two
 // steps and the readback 10.09 ms, now 9.76).
 constexpr uint32_t BATCH_STAGE = 512;  // bodies whose spheres are staged in shared memory
-__global__ void __launch_bounds__(512) k_batch_collide(BatchLaunch B) {
+__global__ void __launch_bounds__(BATCH_WIDE_THREADS) k_batch_collide(BatchLaunch B) {
   __shared__ WorldScope s_scope;
   __shared__ float4 s_sphere[BATCH_STAGE];
   __shared__ uint8_t s_kind[BATCH_STAGE];  // 1: enabled, 2: dynamic
-  __shared__ uint2 s_queue[16][PAIR_QUEUE];
+  __shared__ uint2 s_queue[BATCH_WIDE_THREADS / 32][PAIR_QUEUE];
   const DWorld& w = s_scope.w;
   const StepParams& p = s_scope.p;
   for (;;) {

@@ -305,6 +305,7 @@ cudaError_t launch_batch_solve(const BatchLaunch& b, int blocks, int worldThread
 int batch_collide_blocks_per_sm(int threads);
 int batch_solve_blocks_per_sm(int worldThreads);
 constexpr int BATCH_SOLVE_THREADS = 256;  // the solve's block size (its shared tables assume it)
+constexpr int BATCH_WIDE_THREADS = 512;   // both launches' block size when there are no more worlds than SMs
 constexpr uint32_t BATCH_MAX_WORLD_BODIES = 4096;
 
 // The contact structure of a batched rollout, recorded step by step for the adjoint (avbd_record.cu).

@@ -24,7 +24,6 @@
 namespace avbd {
 
 constexpr int SOLVE_THREADS = 256;
-constexpr int WIDE_SOLVE_THREADS = 512;  // a block a world when there are no more worlds than SMs
 constexpr uint32_t ADJ_SORT_LOCAL = 24;  // adjacency lists up to this long are sorted in local memory
 constexpr long long BARRIER_CYCLES = 4000000000LL;  // about two seconds of SM clock
 
@@ -92,7 +91,7 @@ __device__ bool grid_sync(uint32_t* bar, uint32_t* counters) {
 
 // Exclusive scan of one block's range [lo, hi) in place; returns the range total (all threads).
 __device__ uint32_t block_scan_range(uint32_t* data, uint32_t lo, uint32_t hi) {
-  __shared__ uint32_t warpSums[WIDE_SOLVE_THREADS / 32];
+  __shared__ uint32_t warpSums[BATCH_WIDE_THREADS / 32];
   __shared__ uint32_t s_carry;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) s_carry = 0;
@@ -1823,6 +1822,7 @@ int batch_solve_blocks_per_sm(int worldThreads) {
   if (worldThreads == 32) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_batch_solve_sub<32>, SOLVE_THREADS, 0);
   else if (worldThreads == 64) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_batch_solve_sub<64>, SOLVE_THREADS, 0);
   else if (worldThreads == 128) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_batch_solve_sub<128>, SOLVE_THREADS, 0);
+  else if (worldThreads == BATCH_WIDE_THREADS) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_batch_solve<BATCH_WIDE_THREADS>, BATCH_WIDE_THREADS, 0);
   else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_batch_solve<SOLVE_THREADS>, SOLVE_THREADS, 0);
   return perSm;
 }
@@ -1831,7 +1831,7 @@ cudaError_t launch_batch_solve(const BatchLaunch& b, int blocks, int worldThread
   if (worldThreads == 32) k_batch_solve_sub<32><<<blocks, SOLVE_THREADS, 0, s>>>(b);
   else if (worldThreads == 64) k_batch_solve_sub<64><<<blocks, SOLVE_THREADS, 0, s>>>(b);
   else if (worldThreads == 128) k_batch_solve_sub<128><<<blocks, SOLVE_THREADS, 0, s>>>(b);
-  else if (worldThreads == WIDE_SOLVE_THREADS) k_batch_solve<WIDE_SOLVE_THREADS><<<blocks, WIDE_SOLVE_THREADS, 0, s>>>(b);
+  else if (worldThreads == BATCH_WIDE_THREADS) k_batch_solve<BATCH_WIDE_THREADS><<<blocks, BATCH_WIDE_THREADS, 0, s>>>(b);
   else k_batch_solve<SOLVE_THREADS><<<blocks, SOLVE_THREADS, 0, s>>>(b);
   return cudaGetLastError();
 }
