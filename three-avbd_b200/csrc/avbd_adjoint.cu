@@ -1135,7 +1135,7 @@ __global__ void __launch_bounds__(kThreads, 256 / kThreads) k_adj_backward(const
 // one world's solves run under another's rounds. Forward and backward, 10 iterations, at 64, 128 and
 // 256 threads: 16 worlds of 24 boxes over 12 steps 6.95, 4.59 and 4.45 ms; 1024 of 64 boxes over 8 steps
 // 29.6, 32.7 and 34.4 ms.
-static int blockThreads(int worlds) { return worlds <= 148 ? 256 : worlds <= 296 ? 128 : 64; }
+static int blockThreads(int worlds, int sms) { return worlds <= sms ? 256 : worlds <= 2 * sms ? 128 : 64; }
 
 struct avbd_adjoint {
   int device = 0;
@@ -1187,7 +1187,9 @@ bool aupload(avbd_adjoint* a, const T** dst, const T* src, size_t n) {
 // The replay's working buffers, checkpoints, snapshots and cotangents (D's sizes set)
 bool adjAllocWork(avbd_adjoint* a) {
   AdjDev& D = a->d;
-  a->threads = blockThreads(D.W);
+  int sms = 0;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, a->device) != cudaSuccess) return false;
+  a->threads = blockThreads(D.W, sms);
   // a kernel's limit is the process's, not the handle's: the same for every handle, whatever its points
   const int bytes = int(adjSharedBytes(a->threads, ADJ_MAX_POINTS));
   for (const void* k : {a->forwardKernel(), a->backwardKernel()})

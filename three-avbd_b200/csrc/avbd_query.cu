@@ -629,9 +629,9 @@ int avbd_raycast(avbd_world* w, const avbd_ray* rays, uint32_t n, const uint32_t
     // rays a block: enough blocks for two an SM, a warp a ray at the least; still fewer than SMs: a quarter
     // of the bodies each
     uint32_t chunk = RAY_CHUNK, chunks = std::max(1u, grid_for(w->n, chunk));
-    const uint32_t tile = std::min(RAY_TILE, std::max(RAY_WARPS, grid_for(uint32_t(uint64_t(n) * chunks / 296u), RAY_WARPS) * RAY_WARPS));
+    const uint32_t tile = std::min(RAY_TILE, std::max(RAY_WARPS, grid_for(uint32_t(uint64_t(n) * chunks / uint32_t(2 * w->sms)), RAY_WARPS) * RAY_WARPS));
     const uint32_t tiles = grid_for(n, tile);
-    if (chunks > 1u && chunks * tiles < 148u) {
+    if (chunks > 1u && chunks * tiles < uint32_t(w->sms)) {
       chunk = RAY_CHUNK / 4u;
       chunks = grid_for(w->n, chunk);
     }
