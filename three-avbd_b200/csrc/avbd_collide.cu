@@ -867,8 +867,8 @@ __device__ bool sphereBox(const Box& S, const Box& X, float4 qX, float3& onSpher
 // A pair with a hull on either side (the other a hull, a box or a sphere) collides here: SAT over
 // both shapes' face normals by support points and the edge pairs whose Gauss-map arcs cross
 // (a warp a pair, below), then the incident face clipped by the reference face's side planes, or
-// the closest points of two edges. A box takes part as a hull of its own topology. These run one
-// thread per pair with their clip polygons in local memory, kept out of the box path (noinline).
+// the closest points of two edges. A box takes part as a hull of its own topology. A sphere's
+// pair runs on one thread, kept out of the box path (noinline).
 constexpr uint32_t NO_HULL = 0xffffffffu, MAX_CLIP = 64;
 constexpr float SHAPE_HULL_F = 3.0f;
 __constant__ uint8_t BOX_FACE_VERTS[24] = {1, 3, 7, 5, 0, 2, 6, 4, 2, 3, 7, 6, 0, 1, 5, 4, 4, 5, 7, 6, 0, 1, 3, 2};
@@ -971,117 +971,6 @@ struct EdgeQuery {
   float3 n;
   bool valid;
 };
-__device__ inline uint32_t clipHull(const float3* src, uint32_t n, float3* dst, float3 pn, float offset) {  // wgsl-hull.ts:186-204
-  if (n == 0u) return 0u;
-  uint32_t count = 0;
-  float3 a = src[n - 1u];
-  float da = dot3(pn, a) - offset;
-  for (uint32_t i = 0; i < n; i++) {
-    float3 b = src[i];
-    float db = dot3(pn, b) - offset;
-    if ((da <= PLANE_EPSILON) != (db <= PLANE_EPSILON)) {
-      float t = 0.0f;
-      if (fabsf(da - db) > SAT_AXIS_EPSILON) t = fminf(fmaxf(da / (da - db), 0.0f), 1.0f);
-      if (count < MAX_CLIP) dst[count++] = a + (b - a) * t;
-    }
-    if (db <= PLANE_EPSILON && count < MAX_CLIP) dst[count++] = b;
-    a = b;
-    da = db;
-  }
-  return count;
-}
-// Face contact (wgsl-hull.ts:207-291): the other shape's face clipped to the reference face
-__device__ __noinline__ void hullFaceContact(const DWorld& w, const Poly& A, const Poly& B, bool refIsA, uint32_t refFace, Found& found) {
-  const Poly& R = refIsA ? A : B;
-  const Poly& I = refIsA ? B : A;
-  float4 plane = facePlane(w, R, refFace);
-  float3 rn = make_float3(plane.x, plane.y, plane.z);
-  uint32_t deepest = 0;
-  float low = 3.4e38f;
-  for (uint32_t v = 0; v < I.nv; v++) {
-    float d = dot3(vert(w, I, v), rn);
-    if (d < low) {
-      low = d;
-      deepest = v;
-    }
-  }
-  uint32_t inc = 0;
-  float least = 3.4e38f;
-  for (uint32_t f = 0; f < I.nf; f++) {
-    bool touches = false;
-    uint32_t cnt = faceVertCount(w, I, f);
-    for (uint32_t j = 0; j < cnt; j++)
-      if (faceVert(w, I, f, j) == deepest) {
-        touches = true;
-        break;
-      }
-    if (!touches) continue;
-    float4 pf = facePlane(w, I, f);
-    float d = dot3(make_float3(pf.x, pf.y, pf.z), rn);
-    if (d < least) {
-      least = d;
-      inc = f;
-    }
-  }
-  float3 poly[MAX_CLIP], tmp[MAX_CLIP];
-  uint32_t n = min(faceVertCount(w, I, inc), MAX_CLIP);
-  for (uint32_t j = 0; j < n; j++) poly[j] = vert(w, I, faceVert(w, I, inc, j));
-  const uint32_t k = faceVertCount(w, R, refFace);
-  float3 centre = make_float3(0.0f, 0.0f, 0.0f);
-  for (uint32_t j = 0; j < k; j++) centre = centre + vert(w, R, faceVert(w, R, refFace, j));
-  centre = centre / (float)k;
-  for (uint32_t j = 0; j < k && n > 0u; j++) {
-    float3 v0 = vert(w, R, faceVert(w, R, refFace, j));
-    float3 v1 = vert(w, R, faceVert(w, R, refFace, (j + 1u) % k));
-    float3 sd = cross3(v1 - v0, rn);
-    float l = len3(sd);
-    if (l < SAT_AXIS_EPSILON) continue;
-    sd = sd / l;
-    if (dot3(sd, centre - v0) > 0.0f) sd = -sd;
-    n = clipHull(poly, n, tmp, sd, dot3(sd, v0));
-    for (uint32_t m = 0; m < n; m++) poly[m] = tmp[m];
-  }
-  float depth[MAX_CLIP];
-  uint32_t index[MAX_CLIP];
-  bool chosen[MAX_CLIP];
-  uint32_t keep = 0;
-  for (uint32_t m = 0; m < n; m++) {
-    float dist = dot3(rn, poly[m]) - plane.w;
-    if (dist <= PLANE_EPSILON) {
-      tmp[keep] = poly[m];
-      depth[keep] = dist;
-      index[keep] = m;
-      chosen[keep] = false;
-      keep++;
-    }
-  }
-  const uint32_t prefix = ((refIsA ? AXIS_FACE_A : AXIS_FACE_B) << 24) | (min(refFace, 255u) << 16) | (min(inc, 255u) << 8);
-  for (uint32_t c = 0; c < min(keep, (uint32_t)MAX_CONTACTS); c++) {
-    uint32_t pick = 0;
-    float bestScore = -3.4e38f;
-    for (uint32_t m = 0; m < keep; m++) {
-      if (chosen[m]) continue;
-      float score = -depth[m];
-      if (c > 0u) {
-        score = 3.4e38f;
-        for (uint32_t o = 0; o < keep; o++)
-          if (chosen[o]) score = fminf(score, dot3(tmp[m] - tmp[o], tmp[m] - tmp[o]));
-      }
-      if (score > bestScore) {
-        bestScore = score;
-        pick = m;
-      }
-    }
-    chosen[pick] = true;
-    float3 pp = tmp[pick];
-    float3 onRef = pp - rn * depth[pick];
-    addFound(found, refIsA ? onRef : pp, refIsA ? pp : onRef, prefix | min(index[pick], 255u));
-  }
-  if (found.count == 0u) {
-    float3 nAB = refIsA ? rn : -rn;
-    addFound(found, polySupport(w, A, nAB), polySupport(w, B, -nAB), prefix);
-  }
-}
 // Edge contact (wgsl-hull.ts:293-315): closest points of the two edges
 __device__ inline void hullEdgeContact(const DWorld& w, const Poly& A, const Poly& B, const EdgeQuery& q, Found& found) {
   uint4 ea = edgeOf(w, A, q.ea), eb = edgeOf(w, B, q.eb);
@@ -1191,6 +1080,7 @@ __device__ inline void warpArgMax(float& v, uint32_t& i) {
 // A warp's shared memory: both shapes' vertices in their frames, then, one after the other, a tile of
 // B's edges and the clipping's polygons.
 constexpr uint32_t HULL_VERTS = AVBD_MAX_HULL_VERTICES, EDGE_TILE = 32;
+static_assert(HULL_VERTS <= 32 && HULL_VERTS <= MAX_CLIP, "a lane a vertex; a face's corners fit the clip");
 struct HullScratch {
   float4 verts[2][HULL_VERTS];
   union {
@@ -1215,6 +1105,7 @@ __device__ inline float3 supportStaged(const Poly& P, const float4* verts, float
     return P.c + qrotate(P.q, make_float3(l.x >= 0.0f ? P.h.x : -P.h.x, l.y >= 0.0f ? P.h.y : -P.h.y, l.z >= 0.0f ? P.h.z : -P.h.z));
   float best = -3.4e38f;
   float3 at = make_float3(0.0f, 0.0f, 0.0f);
+#pragma unroll 1
   for (uint32_t v = 0; v < P.nv; v++) {
     float3 q = f3(verts[v]);
     float s = dot3(q, l);
@@ -1323,18 +1214,14 @@ __device__ inline EdgeQuery queryEdgesWarp(const DWorld& w, const Poly& A, const
                     : make_float3(0.0f, 0.0f, 0.0f);
   return out;
 }
-// hullFaceContact with its loops over the lanes: every vertex, face and polygon corner is computed as
-// the sequential loops compute it, argmins keep the first of equals, and the clipped corners keep
-// their order (places by ballots), so the contacts are the same bit for bit. Faces of more than
-// MAX_CLIP corners take the sequential form. Contacts into lane 0's `found`.
+// Face contact (wgsl-hull.ts:186-291): the other shape's face clipped to the reference face, its loops
+// over the lanes. Every vertex, face and polygon corner is computed as the sequential loops there compute
+// it, argmins keep the first of equals, and the clipped corners keep their order (places by ballots), so
+// the contacts are the sequential ones bit for bit. Contacts into lane 0's `found`.
 __device__ void hullFaceContactWarp(const DWorld& w, const Poly& A, const Poly& B, bool refIsA, uint32_t refFace, uint32_t lane, HullScratch& S, Found& found) {
   const Poly& R = refIsA ? A : B;
   const Poly& I = refIsA ? B : A;
-  const uint32_t k = faceVertCount(w, R, refFace);
-  if (k > MAX_CLIP) {
-    if (lane == 0u) hullFaceContact(w, A, B, refIsA, refFace, found);
-    return;
-  }
+  const uint32_t k = faceVertCount(w, R, refFace);  // at most HULL_VERTS
   const uint32_t below = (1u << lane) - 1u;
   float4 plane = facePlane(w, R, refFace);
   float3 rn = make_float3(plane.x, plane.y, plane.z);
@@ -1662,9 +1549,11 @@ __device__ __forceinline__ void writeManifold(const DWorld& w, const StepParams&
 
 // The deferred hull pairs, one warp each: SAT, the contacts (above) and then a lane a point. With the
 // contacts built and written by one lane and every edge pair's normals loaded and rotated anew, 4000
-// hulls heaped among chains (21600 pairs) took a step of 1246 us, now 817.
+// hulls heaped among chains (21600 pairs) took a step of 1246 us, now 751. Five blocks an SM, at 96
+// registers, and the support loop rolled: a step and the wait for it 755; with four blocks at 117
+// registers 808, with six 825, with the loop unrolled 798.
 constexpr uint32_t HULL_THREADS = 128;
-__global__ void __launch_bounds__(HULL_THREADS) k_hull_narrowphase(DWorld w, StepParams p) {
+__global__ void __launch_bounds__(HULL_THREADS, 5) k_hull_narrowphase(DWorld w, StepParams p) {
   __shared__ HullScratch s_scratch[HULL_THREADS / 32];
   HullScratch& S = s_scratch[threadIdx.x >> 5];
   const uint32_t lane = threadIdx.x & 31u;
