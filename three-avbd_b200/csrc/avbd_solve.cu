@@ -794,10 +794,9 @@ __device__ __forceinline__ void stWord(float4* p, float x, float y, float z, uin
   asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p), "l"(lo), "l"(hi) : "memory");
 }
 __device__ __forceinline__ uint32_t tagOf(float4 v) { return __float_as_uint(v.w); }
-// Uses the parts of a polled word that its reader has no need of, always false (no tag has every bit set):
-// with a part unused the assembler narrows the access to several smaller ones, and a tag could arrive with
-// an older value. A word that is read without a look at its tag may be narrowed.
-__device__ __forceinline__ bool brokenWord(float4 v) { return (__float_as_uint(v.y) & __float_as_uint(v.z) & tagOf(v)) == 0xffffffffu; }
+// Uses the parts of a polled word that its reader has no need of, always false: with a part unused the
+// assembler narrows the access to several smaller ones, and a tag could arrive with an older value.
+__device__ __forceinline__ bool brokenWord(float4 v) { return (__float_as_uint(v.y) & __float_as_uint(v.z)) == 0xffffffffu; }
 
 // A body's four words: displacement | 2 vec r | rotation x y z | rotation w, r's w, a filler. Eight bodies'
 // first words lie together, then their second ones and so on: bodies that are near one another in number
@@ -1167,9 +1166,7 @@ __device__ __forceinline__ bool flowLanes(const DWorld& w, const StepParams& p, 
         }
         continue;
       }
-      // The partner's words are as they were read above, so no tag is looked at: it moves again only after
-      // this row's tag (one of the same colour may have, and then either result serves). The row's own words
-      // were last written by this lane.
+      // the partner's words are as they were read above: it moves again only after this row's tag
       FlowRow f;
       issueRow(w, p, inc, f);
       PointView v;
