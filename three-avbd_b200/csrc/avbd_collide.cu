@@ -1105,7 +1105,7 @@ __device__ inline float3 supportStaged(const Poly& P, const float4* verts, float
     return P.c + qrotate(P.q, make_float3(l.x >= 0.0f ? P.h.x : -P.h.x, l.y >= 0.0f ? P.h.y : -P.h.y, l.z >= 0.0f ? P.h.z : -P.h.z));
   float best = -3.4e38f;
   float3 at = make_float3(0.0f, 0.0f, 0.0f);
-#pragma unroll 1
+#pragma unroll 2
   for (uint32_t v = 0; v < P.nv; v++) {
     float3 q = f3(verts[v]);
     float s = dot3(q, l);
@@ -1549,9 +1549,10 @@ __device__ __forceinline__ void writeManifold(const DWorld& w, const StepParams&
 
 // The deferred hull pairs, one warp each: SAT, the contacts (above) and then a lane a point. With the
 // contacts built and written by one lane and every edge pair's normals loaded and rotated anew, 4000
-// hulls heaped among chains (21600 pairs) took a step of 1246 us, now 751. Five blocks an SM, at 96
-// registers, and the support loop rolled: a step and the wait for it 755; with four blocks at 117
-// registers 808, with six 825, with the loop unrolled 798.
+// hulls heaped among chains (21600 pairs) took a step of 1246 us, now 751. The kernel is bound by instruction
+// fetch where pairs fill the SMs, by a warp's own chain where they do not: the support loop is unrolled by two
+// (such worlds of 4000 and of 150 hulls, three at once, a step each: 726 and 131 us; rolled 724, 133; by eight
+// 763, 132). Five blocks an SM, at 96 registers (four at 117 registers, rolled: 7 % slower; six: 9 %).
 constexpr uint32_t HULL_THREADS = 128;
 __global__ void __launch_bounds__(HULL_THREADS, 5) k_hull_narrowphase(DWorld w, StepParams p) {
   __shared__ HullScratch s_scratch[HULL_THREADS / 32];
@@ -1600,7 +1601,7 @@ __global__ void __launch_bounds__(128) k_narrowphase(DWorld w, StepParams p) {
 // BATCH_STAGE bodies the test runs on spheres in shared memory and the pairs that pass it get the full
 // test on full warps: a thread a pair read seven scattered words for every test and ran the full one on
 // the one or two lanes of a warp that came to it (96 worlds a step 597 us, now 494; 4096 worlds, two
-// steps and the readback 10.09 ms, now 9.76).
+// steps and the readback: see WorldScope).
 constexpr uint32_t BATCH_STAGE = 512;  // bodies whose spheres are staged in shared memory
 __global__ void __launch_bounds__(BATCH_WIDE_THREADS) k_batch_collide(BatchLaunch B) {
   __shared__ WorldScope s_scope;
