@@ -782,7 +782,8 @@ static_assert(B_ROWS + MAX_COLORS <= BUCKET_WORDS, "bucket words");
 // second round trip to L2 after it. The sweep is a chain of colours times iterations, each link as long
 // as it takes one body's result to reach the next: with a release store of a count and acquire loads of
 // it, which also emptied L1 of the rows' fixed parts each time, 48 boxes took 127 us of sweep, 3001
-// bodies 231 and 100000 1155; with tagged words 96, 141 and 998 (a B200, 10 iterations).
+// bodies 231 and 100000 1155; with tagged words 96, 141 and 998 (a B200, 10 iterations, a world alone on it:
+// several worlds' steps on their own streams overlap, and then a small one's pass is a third as long).
 __device__ __forceinline__ float4 ldWord(const float4* p) {
   unsigned long long lo, hi;
   asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
@@ -794,8 +795,10 @@ __device__ __forceinline__ void stWord(float4* p, float x, float y, float z, uin
   asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p), "l"(lo), "l"(hi) : "memory");
 }
 __device__ __forceinline__ uint32_t tagOf(float4 v) { return __float_as_uint(v.w); }
-// Uses the parts of a polled word that its reader has no need of, always false: with a part unused the
-// assembler narrows the access to several smaller ones, and a tag could arrive with an older value.
+// Uses the parts of a polled word that its reader has no need of, always false (a NaN that the sweep writes
+// is the hardware's, 0x7fffffff): with a part unused the assembler narrows the access to several smaller
+// ones, and a tag could arrive with an older value. A word that is read without a look at its tag may be
+// narrowed. (The tag as a third part here: worlds of joints 10 us a solve longer, 216 to 227 with 50 chains.)
 __device__ __forceinline__ bool brokenWord(float4 v) { return (__float_as_uint(v.y) & __float_as_uint(v.z)) == 0xffffffffu; }
 
 // A body's four words: displacement | 2 vec r | rotation x y z | rotation w, r's w, a filler. Eight bodies'
@@ -1166,7 +1169,9 @@ __device__ __forceinline__ bool flowLanes(const DWorld& w, const StepParams& p, 
         }
         continue;
       }
-      // the partner's words are as they were read above: it moves again only after this row's tag
+      // The partner's words are as they were read above, so no tag is looked at: it moves again only after
+      // this row's tag (one of the same colour may have, and then either result serves). The row's own words
+      // were last written by this lane.
       FlowRow f;
       issueRow(w, p, inc, f);
       PointView v;
@@ -1849,7 +1854,8 @@ int solve_grid_blocks(int device) {
 // SM with all its registers is faster (5000 bodies: a solve of 227 us against 262), and fewer blocks
 // meet sooner at the barriers between the topology's phases, so long as a colour's rows still get a
 // lane each (48 boxes, a block for 16 bodies: 121; for 32: 134; for 64: 168). Past it the chunks outnumber
-// the warps and two blocks an SM win (12000 bodies: 298 against 336, 16000: 350 against 410).
+// the warps and two blocks an SM win (12000 bodies: 298 against 336, 16000: 350 against 410). All of a
+// world alone.
 constexpr uint32_t SMALL_SOLVE = 8192;
 constexpr uint32_t CLEAR_WORDS = 256;
 cudaError_t launch_topology_solve(const DWorld& w, const StepParams& p, int blocks, int maxBlocks, int sms, cudaStream_t s) {
